@@ -17,6 +17,7 @@
 #include "bp_common.cuh"
 #include "bp_kernels.cuh"
 #include "bp_host.h"
+#include "bp_tmem.cuh"
 
 namespace bp_host {
 
@@ -90,7 +91,8 @@ constexpr CfgDesc cfg_desc() {
 }
 constexpr CfgDesc kCfgDesc[kNumConfigs] = {cfg_desc<0>(), cfg_desc<1>(), cfg_desc<2>(),
                                            cfg_desc<3>(), cfg_desc<4>(), cfg_desc<5>(),
-                                           cfg_desc<6>(), cfg_desc<7>(), cfg_desc<8>()};
+                                           cfg_desc<6>(), cfg_desc<7>(), cfg_desc<8>(),
+                                           {4, 16, 16, 4, 1, 64, 1}};
 
 inline const CfgDesc& cfg_of(int cfg) {
   return kCfgDesc[(cfg >= 0 && cfg < kNumConfigs) ? cfg : 0];
@@ -102,7 +104,8 @@ inline int cfg_blocks_per_tile(int cfg) { return kTileSources / cfg_of(cfg).k; }
 // Preferred config per (storage, reduce); -1 = built-in default.
 std::atomic<int> g_cfg_choice[3][2] = {{{-1}, {-1}}, {{-1}, {-1}}, {{-1}, {-1}}};
 
-int pick_config(int storage, bool maxred) {
+// The caller's choice of shape, or -1.
+int chosen_config(int storage, bool maxred) {
   if (const char* v = std::getenv("BEAMPOWER_B200_KERNEL_CONFIG")) {
     const int c = std::atoi(v);
     if (c >= 0 && c < kNumConfigs) return c;
@@ -111,12 +114,7 @@ int pick_config(int storage, bool maxred) {
     const int c = g_cfg_choice[storage][maxred ? 1 : 0].load();
     if (c >= 0 && c < kNumConfigs) return c;
   }
-  // Built-in defaults, measured on B200 (400,000 sources x 60 stations x
-  // 180,000 samples, reduce='max'): FP32 storage runs fastest with config 8
-  // (32-source blocks, 721 ms; config 3 741 ms, config 0 757 ms), 16-bit
-  // storage with config 2 (16 warps x 4 sources x 16 samples, two stations
-  // per ring stage; FP16 471 ms, BF16 510 ms).
-  return storage == BP_STORAGE_F32 ? 8 : 2;
+  return -1;
 }
 
 }  // namespace
@@ -130,6 +128,8 @@ struct bp_table {
   int32_t* delays;   // (N, S, P), direct kernel only
   float* weights;    // (N, S), direct kernel only
   int* status;       // kernel status word
+  double mean_spread;  // mean span of the used (tile, station, phase) windows
+  bool real_weights;   // some weight is neither 0 nor 1
   int device;
   cudaStream_t stream;
 };
@@ -145,7 +145,7 @@ __global__ void init_stats_kernel(int* stats, int* status) {
     stats[bp::kStatNonFinite] = 0;
     stats[bp::kStatMinLoAligned] = INT_MAX;
     stats[bp::kStatWideTile] = 0;
-    stats[7] = 0;
+    for (int i = 7; i < bp::kStatCount; ++i) stats[i] = 0;
     *status = 0;
   }
 }
@@ -285,6 +285,14 @@ int launch_window(int cfg, int P, bool checked, int storage, const bp::LaunchArg
     case 6: return launch_window_c<6, MAXRED>(P, checked, storage, a, batch, blocks, dev, st);
     case 7: return launch_window_c<7, MAXRED>(P, checked, storage, a, batch, blocks, dev, st);
     case 8: return launch_window_c<8, MAXRED>(P, checked, storage, a, batch, blocks, dev, st);
+    case kTmemConfig:
+      if (storage == BP_STORAGE_F32)
+        return launch_tmem<MAXRED, BP_STORAGE_F32>(P, a, batch, blocks, dev, st);
+      if (storage == BP_STORAGE_BF16)
+        return launch_tmem<MAXRED, BP_STORAGE_BF16>(P, a, batch, blocks, dev, st);
+      if (storage == BP_STORAGE_F16)
+        return launch_tmem<MAXRED, BP_STORAGE_F16>(P, a, batch, blocks, dev, st);
+      return fail(BP_ERR_INVALID_ARGUMENT, "unknown storage %d", storage);
     default: return launch_window_c<0, MAXRED>(P, checked, storage, a, batch, blocks, dev, st);
   }
 }
@@ -330,7 +338,75 @@ size_t staged_smem_bytes(int cfg, int P, bool maxred, int rowcap, int max_active
   }
 }
 
+// Shared memory of the tensor-memory kernel.
+size_t tmem_smem_bytes(int P, bool maxred, int max_rows, int max_active, int n_stage) {
+  auto f = [&](auto tag) -> size_t {
+    constexpr int PP = decltype(tag)::value;
+    return maxred ? bp::tm_layout<PP, true>(max_rows, max_active, n_stage).total
+                  : bp::tm_layout<PP, false>(max_rows, max_active, n_stage).total;
+  };
+  switch (P) {
+    case 1: return f(std::integral_constant<int, 1>{});
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 3: return f(std::integral_constant<int, 3>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+  }
+  return SIZE_MAX;
+}
+
+// Ring stages (4 to 2) the tensor-memory kernel can have; 0 when two do not
+// fit, one window exceeds the TMEM columns or the planes' grid its limit.
+int tmem_stages(int S, int P, bool maxred, int max_spread, int max_active, int storage,
+                int dev) {
+  // a window may begin 15 samples past a row's start; at most a chunk less one
+  // sample of them stays in
+  const bool f32 = storage == BP_STORAGE_F32;
+  if (bp::tm_cols(0, max_spread + bp::tm_chunk(f32), f32) > bp::kTmCols || S * P * 2 > 65535)
+    return 0;
+  const int max_rows = bp::tm_rows(max_spread + 15);
+  for (int n = bp::kTmMaxStage; n >= 2; --n)
+    if (tmem_smem_bytes(P, maxred, max_rows, max_active, n) <= (size_t)device_smem_optin(dev))
+      return n;
+  return 0;
+}
+
+// Bytes of a record's traces as planes; traces -> planes.
+size_t planes_bytes(int S, int P, size_t pitch) {
+  return (size_t)S * P * 64 * (size_t)bp::tm_plane_rows((long long)pitch);
+}
+int fill_planes(int S, int P, int storage, const void* traces, size_t pitch, void* planes,
+                cudaStream_t st) {
+  const bool f32 = storage == BP_STORAGE_F32;
+  const long long chunks = bp::tm_plane_rows((long long)pitch) * (f32 ? 4 : 2);
+  const dim3 grid((unsigned)((chunks + 255) / 256), (unsigned)(S * P * (f32 ? 1 : 2)));
+  const auto* in = static_cast<const uint4*>(traces);
+  auto* out = static_cast<uint4*>(planes);
+  if (f32) bp::planes_kernel<true><<<grid, 256, 0, st>>>(in, (long long)pitch, out);
+  else bp::planes_kernel<false><<<grid, 256, 0, st>>>(in, (long long)pitch, out);
+  BP_LAUNCHED("planes_kernel");
+  return BP_OK;
+}
+
+// A plain call's planes: stream-ordered scratch, given back after the kernel.
+struct PlanesScratch {
+  void* p = nullptr;
+  cudaStream_t s = nullptr;
+  // false: no memory for them (the staged kernel needs none)
+  bool get(size_t bytes, cudaStream_t st) {
+    s = st;
+    if (cudaMallocAsync(&p, bytes, st) == cudaSuccess) return true;
+    p = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  ~PlanesScratch() {
+    if (p) cudaFreeAsync(p, s);
+  }
+};
+
 int rowcap_for(const bp_table* t, int cfg) {
+  if (cfg == kTmemConfig)
+    return bp::tm_rows(t->info.max_spread + 15);  // plane rows
   return (int)bp::align_up_sz((size_t)(cfg_time_tile(cfg) + t->info.max_spread + 1),
                               bp::kAlign);
 }
@@ -349,7 +425,11 @@ int device_smem_per_sm(int dev) {
 // fits a block, or the blocks per SM the shape is built for do not fit an
 // SM (a two-block shape left at one block per SM runs at half its
 // occupancy).  Without the max reduction the buffer is empty.
+// The tensor-memory kernel: its ring stages in the place of the rows.
 int rows_for(const bp_table* t, int c, int storage, bool maxred) {
+  if (c == kTmemConfig)
+    return tmem_stages(t->dev.S, t->dev.P, maxred, t->info.max_spread,
+                       std::max(1, t->info.max_active), storage, t->device);
   const int ws = cfg_of(c).ws;
   const int minb = cfg_of(c).minb;
   for (int rows : {ws, 1}) {
@@ -369,26 +449,60 @@ bool config_fits(const bp_table* t, int c, int storage, bool maxred) {
 
 // Fallback order when the chosen shape does not fit a table, fastest first
 // (measured on the 400,000-source workload).
-const int kOrderF32[kNumConfigs] = {8, 3, 0, 1, 2, 4, 5, 6, 7};
-const int kOrder16[kNumConfigs] = {2, 1, 6, 7, 0, 5, 4, 3, 8};
+const int kOrderF32[kStagedConfigs] = {8, 3, 0, 1, 2, 4, 5, 6, 7};
+const int kOrder16[kStagedConfigs] = {2, 1, 6, 7, 0, 5, 4, 3, 8};
 
-// The preferred config if it serves this table, else the first one of the
-// storage's fallback order that does; config 0 (the smallest) as the last
-// resort.
-int config_for(const bp_table* t, int storage, bool maxred) {
-  const int c = pick_config(storage, maxred);
-  if (config_fits(t, c, storage, maxred)) return c;
+// Whether the tensor-memory kernel is the faster one for a table: FP32 and
+// windows that are narrow on average (its TMEM fills take (16 + span) / 4
+// copies per station and phase, and wide ones leave TMEM room for fewer).
+// Measured against the staged shape 8 (16,000 sources, 30 stations, 18,000
+// samples; ms, staged | tensor memory):
+//   max, weights 0 / 1:  span 35: 2.37 | 1.51, 65: 2.35 | 1.61,
+//                        110: 2.35 | 1.97, 139: 2.35 | 2.23
+//   max, any weights:    65: 2.74 | 2.45, 89: 2.75 | 2.69, 110: 2.75 | 2.81
+//   whole response, 0 / 1 (6,250 sources): 50: 0.99 | 0.78, 89: 0.99 | 0.90,
+//                        120: 0.99 | 0.98, 147: 0.99 | 1.11
+//   1 phase, max, 0 / 1: 50: 1.43 | 1.00, 122: 1.41 | 1.17
+//   3 phases, max, 0 / 1: 50: 4.03 | 2.88, 89: 3.45 | 3.61
+// 16-bit storage halves what the staged shapes read and keeps them ahead
+// (FP16, span 65: 1.47 | 2.27).
+bool prefers_tmem(const bp_table* t, int storage, bool maxred) {
+  if (storage != BP_STORAGE_F32) return false;
+  double limit = t->real_weights ? 90.0 : 145.0;
+  if (t->dev.P > 2) limit = std::min(limit, 80.0);
+  if (!maxred) limit -= 30.0;
+  return t->mean_spread <= limit;
+}
+
+// The caller's choice if it serves this table; else the tensor-memory kernel
+// where it is the faster one; else the first shape of the storage's order
+// that serves the table; config 0 (the smallest) as the last resort.
+// staged_only: non-finite weights under the flexible rule, or no memory for
+// the planes.
+int config_for(const bp_table* t, int storage, bool maxred, bool staged_only = false) {
+  const int c = chosen_config(storage, maxred);
+  if (c >= 0 && !(staged_only && c == kTmemConfig) && config_fits(t, c, storage, maxred))
+    return c;
+  if (!staged_only && prefers_tmem(t, storage, maxred) &&
+      config_fits(t, kTmemConfig, storage, maxred))
+    return kTmemConfig;
   const int* order = storage == BP_STORAGE_F32 ? kOrderF32 : kOrder16;
-  for (int i = 0; i < kNumConfigs; ++i)
+  for (int i = 0; i < kStagedConfigs; ++i)
     if (config_fits(t, order[i], storage, maxred)) return order[i];
   return 0;
+}
+
+// Rows of the max buffer, or the tensor-memory kernel's ring stages.
+void set_fit(bp::LaunchArgs& a, int cfg, int rows) {
+  a.red_rows = std::max(1, rows);
+  a.n_stage = cfg == kTmemConfig ? rows : 0;
 }
 
 // Whether some staged shape serves table `t` with this storage and reduction
 // (tables too wide for every shape's ring run the direct kernel).
 bool staged_serves(const bp_table* t, int storage, bool maxred) {
   if (!t->info.uses_window_kernel) return false;
-  for (int c = 0; c < kNumConfigs; ++c)
+  for (int c = 0; c < kStagedConfigs; ++c)
     if (config_fits(t, c, storage, maxred)) return true;
   return false;
 }
@@ -447,19 +561,29 @@ int run_staged(const bp_table* t, const void* traces, int storage, const float* 
   r.beam = beam;
   r.ldb = (long long)ldb;
   const bool maxred = keys != nullptr;
-  const int cfg = config_for(t, storage, maxred);
+  const bool checked = out_of_bounds && t->info.any_nonfinite;
+  int cfg = config_for(t, storage, maxred, checked);
+  PlanesScratch planes;
+  if (cfg == kTmemConfig && T > 0) {
+    if (planes.get(planes_bytes(t->dev.S, t->dev.P, pitch), st)) {
+      if (int rc = fill_planes(t->dev.S, t->dev.P, storage, traces, pitch, planes.p, st))
+        return rc;
+      r.planes = static_cast<const unsigned char*>(planes.p);
+    } else {
+      cfg = config_for(t, storage, maxred, true);
+    }
+  }
   const int tt = cfg_time_tile(cfg);
   const int n_tt = (int)((T + tt - 1) / tt);
   const int n_btiles = t->dev.n_tiles * cfg_blocks_per_tile(cfg);
   a.tiles_per_chunk = choose_tiles_per_chunk(n_tt, n_btiles, t->device);
   a.rowcap = rowcap_for(t, cfg);
   a.max_active = std::max(1, t->info.max_active);
-  a.red_rows = std::max(1, rows_for(t, cfg, storage, maxred));
+  set_fit(a, cfg, rows_for(t, cfg, storage, maxred));
   a.status = t->status;
   if (n_tt == 0) return BP_OK;
   const long long blocks =
       (long long)((n_tt + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
-  const bool checked = out_of_bounds && t->info.any_nonfinite;
   if (maxred)
     return launch_window<true>(cfg, t->dev.P, checked, storage, a, false, blocks, t->device, st);
   return launch_window<false>(cfg, t->dev.P, checked, storage, a, false, blocks, t->device, st);
@@ -724,6 +848,13 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
   in.max_spread = stats[bp::kStatMaxSpread];
   in.max_active = stats[bp::kStatMaxActive];
   in.any_nonfinite = stats[bp::kStatNonFinite];
+  {
+    unsigned long long rows = 0, sum = 0;
+    std::memcpy(&rows, stats + bp::kStatSpreadRows, 8);
+    std::memcpy(&sum, stats + bp::kStatSpreadSum, 8);
+    t->real_weights = stats[bp::kStatReal] != 0;
+    t->mean_spread = rows ? (double)sum / (double)rows : 0.0;
+  }
   // The staged kernel serves the table when some shape holds its windows
   // with FP32 storage (the smallest ring).  16-bit storage keeps four copies
   // of every window and may fit no shape where FP32 does; such calls expand
@@ -1344,6 +1475,10 @@ struct bp_batch {
   int max_active;
   int red_rows;
   bool checked;
+  void* planes;                     // tensor-memory kernel: the records' traces as planes
+  std::vector<size_t> planes_at;    // byte offset of each record's planes
+  std::vector<bp_record> records;   // their traces
+  std::vector<int> record_S;
   void* mem;                        // device: tables, records, prefix, keys, srcmm, queue, status
   bp::TableView* d_tables;
   bp::RecordView* d_records;
@@ -1390,14 +1525,56 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   BP_CUDA(cudaGetDevice(&dev));
   retain_pool(dev);
   const int P = tables[0] ? tables[0]->dev.P : 0;
-  // the preferred shape if it serves every table, else the first of the
-  // fallback order that does
-  int cfg = -1;
+  bool any_flexible = false, any_nonfinite = false;
+  for (int r = 0; r < n_records; ++r) any_flexible |= records[r].out_of_bounds != 0;
+  for (int j = 0; j < n_tables; ++j) any_nonfinite |= tables[j] && tables[j]->info.any_nonfinite;
+  const bool checked = any_flexible && any_nonfinite;
+  // the caller's shape if it serves every table, else the tensor-memory
+  // kernel where it is the faster one for every table, its shared memory
+  // holds the widest windows beside the most stations and there is memory for
+  // the records' planes, else the first of the fallback order that serves
+  // every table
+  int n_stage = 0;
+  void* planes = nullptr;
+  const int chosen = chosen_config(storage, true);
+  if (!checked && P >= 1 && P <= 4 && (chosen < 0 || chosen == kTmemConfig)) {
+    bool tmem = true;
+    int S = 0, spread = 0, active = 1;
+    for (int j = 0; j < n_tables && tmem; ++j) {
+      const bp_table* t = tables[j];
+      tmem = t && staged_serves(t, storage, true) && t->dev.P == P && t->device == dev &&
+             (chosen == kTmemConfig || prefers_tmem(t, storage, true));
+      if (!tmem) break;
+      S = std::max(S, t->dev.S);
+      spread = std::max(spread, t->info.max_spread);
+      active = std::max(active, t->info.max_active);
+    }
+    if (tmem) n_stage = tmem_stages(S, P, true, spread, active, storage, dev);
+    if (n_stage) {
+      size_t bytes = 0;
+      for (int r = 0; r < n_records; ++r)
+        if (records[r].table >= 0 && records[r].table < n_tables)
+          bytes += planes_bytes(tables[records[r].table]->dev.S, P, records[r].pitch);
+      if (cudaMallocAsync(&planes, std::max<size_t>(bytes, 16), st) != cudaSuccess) {
+        planes = nullptr;
+        n_stage = 0;
+        cudaGetLastError();
+      }
+    }
+  }
+  struct PlanesGuard {  // until the batch owns them
+    void*& p;
+    cudaStream_t s;
+    ~PlanesGuard() {
+      if (p) cudaFreeAsync(p, s);
+    }
+  } planes_guard{planes, st};
+  int cfg = n_stage ? kTmemConfig : -1;
   {
-    const int pref = pick_config(storage, true);
     const int* order = storage == BP_STORAGE_F32 ? kOrderF32 : kOrder16;
-    for (int i = -1; i < kNumConfigs && cfg < 0; ++i) {
-      const int c = i < 0 ? pref : order[i];
+    for (int i = -1; i < kStagedConfigs && cfg < 0; ++i) {
+      const int c = i < 0 ? chosen : order[i];
+      if (c < 0 || c == kTmemConfig) continue;
       bool all = true;
       for (int j = 0; j < n_tables; ++j)
         if (tables[j] && staged_serves(tables[j], storage, true) &&
@@ -1412,9 +1589,9 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   for (int j = 0; j < n_tables; ++j)
     if (tables[j] && staged_serves(tables[j], storage, true))
       red_rows = std::min(red_rows, std::max(1, rows_for(tables[j], cfg, storage, true)));
+  if (cfg == kTmemConfig) red_rows = n_stage;
   const int tt = cfg_time_tile(cfg);
   int rowcap = 0, max_active = 1;
-  bool any_nonfinite = false;
   std::vector<bp::TableView> tv(n_tables);
   for (int i = 0; i < n_tables; ++i) {
     const bp_table* t = tables[i];
@@ -1427,13 +1604,11 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
     if (t->device != dev) return fail(BP_ERR_INVALID_ARGUMENT, "table %d is on another device", i);
     rowcap = std::max(rowcap, rowcap_for(t, cfg));
     max_active = std::max(max_active, t->info.max_active);
-    any_nonfinite |= t->info.any_nonfinite != 0;
     tv[i] = table_view(t);
   }
   std::vector<bp::RecordView> rv(n_records);
   std::vector<long long> prefix(n_records + 1, 0);
   size_t n_keys = 0, n_srcmm = 0;
-  bool any_flexible = false;
   for (int r = 0; r < n_records; ++r) {
     const bp_record& q = records[r];
     if (q.table < 0 || q.table >= n_tables)
@@ -1446,7 +1621,6 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
     if (!q.traces || !q.beam_max || !q.argmax || (storage != BP_STORAGE_F32 && !q.scales))
       return fail(BP_ERR_INVALID_ARGUMENT, "record %d: NULL pointer", r);
     if (int rc = check_layout(t, q.n_samples, q.lpad, q.pitch)) return rc;
-    any_flexible |= q.out_of_bounds != 0;
     bp::RecordView& v = rv[r];
     v = bp::RecordView{};
     v.traces = q.traces;
@@ -1480,7 +1654,11 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   b->cfg = cfg;
   b->max_active = max_active;
   b->red_rows = red_rows;
-  b->checked = any_flexible && any_nonfinite;
+  b->checked = checked;
+  b->mem = nullptr;
+  b->planes = planes;
+  planes = nullptr;
+  b->records.assign(records, records + n_records);
   b->stream = st;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -1497,7 +1675,8 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   const size_t o_s = take(sizeof(int));
   cudaError_t e = cudaMallocAsync(&b->mem, off, st);
   if (e != cudaSuccess) {
-    delete b;
+    b->mem = nullptr;
+    bp_batch_destroy(b);
     return cuda_fail(e, "cudaMallocAsync(batch)");
   }
   char* base = static_cast<char*>(b->mem);
@@ -1513,10 +1692,17 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
     return rc;
   };
   // keys and delay ranges inside the allocation
-  size_t koff = 0, moff = 0;
+  size_t koff = 0, moff = 0, poff = 0;
   int2* d_srcmm = reinterpret_cast<int2*>(base + o_m);
   for (int r = 0; r < n_records; ++r) {
     rv[r].keys = b->d_keys + koff;
+    if (b->planes) {
+      const int S = tables[rv[r].table]->dev.S;
+      rv[r].planes = static_cast<const unsigned char*>(b->planes) + poff;
+      b->planes_at.push_back(poff);
+      b->record_S.push_back(S);
+      poff += planes_bytes(S, P, records[r].pitch);
+    }
     koff += (size_t)(rv[r].out1 - rv[r].out0);
     if (records[r].station_mask) {
       rv[r].srcmm = d_srcmm + moff;
@@ -1548,6 +1734,12 @@ int bp_batch_run(bp_batch* b, void* stream) {
   cudaStream_t st = as_stream(stream);
   BP_CUDA(cudaMemsetAsync(b->d_keys, 0, std::max<size_t>(b->n_keys, 1) * 8, st));
   BP_CUDA(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned long long), st));
+  if (b->planes)
+    for (int r = 0; r < b->n_records; ++r)
+      if (int rc = fill_planes(b->record_S[r], b->P, b->storage, b->records[r].traces,
+                               b->records[r].pitch,
+                               static_cast<unsigned char*>(b->planes) + b->planes_at[r], st))
+        return rc;
   bp::LaunchArgs a{};
   a.tables = b->d_tables;
   a.records = b->d_records;
@@ -1556,7 +1748,7 @@ int bp_batch_run(bp_batch* b, void* stream) {
   a.next_item = b->d_queue;
   a.rowcap = b->rowcap;
   a.max_active = b->max_active;
-  a.red_rows = b->red_rows;
+  set_fit(a, b->cfg, b->red_rows);
   a.status = b->d_status;
   if (int rc = launch_window<true>(b->cfg, b->P, b->checked, b->storage, a, true, 0, b->device,
                                    st))
@@ -1578,6 +1770,7 @@ int bp_batch_status(bp_batch* b, void* stream, int* status) {
 int bp_batch_destroy(bp_batch* b) {
   if (!b) return BP_OK;
   if (b->mem) cudaFreeAsync(b->mem, b->stream);
+  if (b->planes) cudaFreeAsync(b->planes, b->stream);
   cudaStreamSynchronize(b->stream);
   delete b;
   return BP_OK;
@@ -1625,7 +1818,18 @@ int bp_record_beamform_max_dev(const bp_table* t, const bp_record* q, int storag
   r.out1 = (int)q->out1;
   r.flexible = q->out_of_bounds;
   r.keys = keys;
-  const int cfg = config_for(t, storage, true);
+  const bool checked = q->out_of_bounds && t->info.any_nonfinite;
+  int cfg = config_for(t, storage, true, checked);
+  PlanesScratch planes;
+  if (cfg == kTmemConfig) {
+    if (planes.get(planes_bytes(t->dev.S, t->dev.P, q->pitch), st)) {
+      if (int rc = fill_planes(t->dev.S, t->dev.P, storage, r.traces, q->pitch, planes.p, st))
+        return rc;
+      r.planes = static_cast<const unsigned char*>(planes.p);
+    } else {
+      cfg = config_for(t, storage, true, true);
+    }
+  }
   const int tt = cfg_time_tile(cfg);
   const int tau_first = r.out0 / tt;
   const int n_tt = (r.out1 + tt - 1) / tt - tau_first;
@@ -1633,11 +1837,10 @@ int bp_record_beamform_max_dev(const bp_table* t, const bp_record* q, int storag
   a.tiles_per_chunk = choose_tiles_per_chunk(n_tt, n_btiles, t->device);
   a.rowcap = rowcap_for(t, cfg);
   a.max_active = std::max(1, t->info.max_active);
-  a.red_rows = std::max(1, rows_for(t, cfg, storage, true));
+  set_fit(a, cfg, rows_for(t, cfg, storage, true));
   a.status = t->status;
   const long long blocks =
       (long long)((n_tt + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
-  const bool checked = q->out_of_bounds && t->info.any_nonfinite;
   if (int rc = launch_window<true>(cfg, t->dev.P, checked, storage, a, false, blocks, t->device,
                                    st))
     return rc;
@@ -1699,7 +1902,8 @@ int bp_table_kernel_config(const bp_table* t, int storage, int reduce) {
 
 int bp_get_kernel_config(int storage, int reduce) {
   if (storage < 0 || storage > 2) return 0;
-  return pick_config(storage, reduce == BP_REDUCE_MAX);
+  const int c = chosen_config(storage, reduce == BP_REDUCE_MAX);
+  return c >= 0 ? c : kTmemConfig;
 }
 
 }  // extern "C"

@@ -141,6 +141,40 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same for waits that are part of a kernel's rhythm: a tight loop of 4096
+// tries between looks at the abort flag and the clock.
+__device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, int* status) {
+  unsigned long long start = 0;
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, 0;\n"
+        "WAIT:\n\t"
+        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE;\n\t"
+        "add.u32 n, n, 1;\n\t"
+        "setp.lt.u32 p, n, 4096;\n\t"
+        "@p bra WAIT;\n"
+        "DONE:\n\t"
+        "setp.lt.u32 p, n, 4096;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (*abort_flag) return false;
+    const unsigned long long now = globaltimer_ns();
+    if (start == 0) start = now;
+    if (now - start > kWaitLimitNs) {
+      *abort_flag = 1;
+      if (status) atomicOr(status, kStatusWaitTimeout);
+      return false;
+    }
+  }
+}
+
 // Same with a caller-given limit (diagnostics).
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity,
                                                 unsigned long long limit_ns, int* status) {

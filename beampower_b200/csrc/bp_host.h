@@ -81,7 +81,11 @@ template <> struct KCfg<5> : KShape<16, 2, 32, 2, 1> {};
 template <> struct KCfg<6> : KShape<8, 8, 16, 2, 1> {};
 template <> struct KCfg<7> : KShape<8, 8, 16, 1, 1> {};
 template <> struct KCfg<8> : KShape<16, 2, 16, 2, 1> {};
-constexpr int kNumConfigs = 9;
+// Config 9 is the tensor-memory kernel (bp_tmem.cuh): 16 compute warps x 4
+// sources x 16 samples, one station per ring stage, 1/SM.
+constexpr int kStagedConfigs = 9;
+constexpr int kTmemConfig = 9;
+constexpr int kNumConfigs = 10;
 constexpr int kTileSources = bp::kTableTile;
 
 // Launches the staged kernel of config CFG (plain grid of `blocks` blocks, or
@@ -106,6 +110,20 @@ BP_EXTERN_CFG(6)
 BP_EXTERN_CFG(7)
 BP_EXTERN_CFG(8)
 #undef BP_EXTERN_CFG
+
+// The same for the tensor-memory kernel; instantiated in bp_tmem_*.cu.
+template <bool MAXRED, int STORAGE>
+int launch_tmem(int P, const bp::LaunchArgs& a, bool batch, long long blocks, int dev,
+                cudaStream_t st);
+#define BP_EXTERN_TMEM(S)                                                                  \
+  extern template int launch_tmem<true, S>(int, const bp::LaunchArgs&, bool, long long, int, \
+                                           cudaStream_t);                                  \
+  extern template int launch_tmem<false, S>(int, const bp::LaunchArgs&, bool, long long, int, \
+                                            cudaStream_t);
+BP_EXTERN_TMEM(BP_STORAGE_F32)
+BP_EXTERN_TMEM(BP_STORAGE_BF16)
+BP_EXTERN_TMEM(BP_STORAGE_F16)
+#undef BP_EXTERN_TMEM
 
 }  // namespace bp_host
 

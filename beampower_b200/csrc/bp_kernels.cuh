@@ -74,7 +74,10 @@ enum : int {
   kStatNonFinite = 4,  // a non-zero weight is NaN or inf
   kStatMinLoAligned = 5,
   kStatWideTile = 6,   // a window span does not fit 16-bit offsets
-  kStatCount = 8
+  kStatReal = 7,         // a weight is neither 0 nor 1
+  kStatSpreadRows = 8,  // used (tile, station, phase) windows (64 bits)
+  kStatSpreadSum = 10,  // sum of their spans (64 bits)
+  kStatCount = 12
 };
 
 // Per (tile, station, source) metadata: weight bits and 16-bit offsets.
@@ -123,7 +126,7 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
   // 1. per source: min / max over weighted stations, non-finite weights.
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     const int o = orig_of(k);
-    int mn = INT_MAX, mx = INT_MIN, bad = 0;
+    int mn = INT_MAX, mx = INT_MIN, bad = 0, real = 0;
     if (o >= 0) {
       const int32_t* d = delays + (size_t)o * S * P;
       const float* w = weights + (size_t)o * S;
@@ -131,6 +134,7 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
         const float ws = w[s];
         if (ws == 0.0f) continue;
         if (!isfinite(ws)) bad = 1;
+        real |= ws != 1.0f;
         for (int p = 0; p < P; ++p) {
           const int v = d[s * P + p];
           mn = min(mn, v);
@@ -140,6 +144,7 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
     }
     tb.src_info[(size_t)tile * K + k] = make_int4(o >= 0 ? o + tb.index_base : o, mn, mx, 0);
     if (bad) atomicOr(&tb.stats[kStatNonFinite], 1);
+    if (real) atomicOr(&tb.stats[kStatReal], 1);
   }
   // 2. per (station, phase): window over the tile's weighted sources.
   for (int sp = threadIdx.x; sp < S * P; sp += blockDim.x) {
@@ -159,6 +164,7 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
   __syncthreads();
   // 3. active station list, ascending station index (the summation order).
   if (threadIdx.x == 0) {
+    unsigned long long spread_sum = 0;
     int n = 0, spread_max = 0, mn = INT_MAX, mx = INT_MIN, lo_al_min = INT_MAX, wide = 0;
     for (int s = 0; s < S; ++s) {
       if (lo[s * P] > hi[s * P]) {  // no weighted source in this tile
@@ -176,6 +182,7 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
         tb.st_lo[((size_t)tile * S + n) * P + p] = la;
         tb.st_spread[((size_t)tile * S + n) * P + p] = sp32;
         spread_max = max(spread_max, sp32);
+        spread_sum += (unsigned long long)sp32;
         mn = min(mn, l);
         mx = max(mx, h);
         lo_al_min = min(lo_al_min, la);
@@ -191,6 +198,9 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
     }
     atomicMax(&tb.stats[kStatMaxSpread], spread_max);
     atomicMax(&tb.stats[kStatMaxActive], n);
+    auto* sums = reinterpret_cast<unsigned long long*>(tb.stats);
+    atomicAdd(&sums[kStatSpreadRows / 2], (unsigned long long)(n * P));
+    atomicAdd(&sums[kStatSpreadSum / 2], spread_sum);
     if (wide) atomicOr(&tb.stats[kStatWideTile], 1);
   }
   __syncthreads();
@@ -280,6 +290,13 @@ struct RecordView {
   long long ldb;
   float* beam_max;              // batch launch: decoded outputs [out1 - out0]
   int32_t* argmax;
+  const unsigned char* planes;  // tensor-memory kernel: the traces as planes
+};
+
+// Shared memory of the tensor-memory kernel (bp_tmem.cuh), byte offsets.
+struct TmLayout {
+  int n_stage, plane_bytes;
+  uint32_t red, records, weights, el_src, el_info, st_j, ring, total, reserved[2];
 };
 
 struct LaunchArgs {
@@ -298,6 +315,8 @@ struct LaunchArgs {
   // into with shared-memory atomics -- the host takes 1 when the per-warp
   // rows would not leave room for the table's ring.
   int red_rows;
+  int n_stage;  // tensor-memory kernel: ring stages
+  TmLayout tm;  // filled at its launch
   int* status;
 };
 

@@ -218,8 +218,9 @@ typedef struct bp_batch bp_batch;
 /* One record alone (no batch): the plain staged launch over the record's
  * output range, global time origin included; this is what a streamed chunk
  * with its carried samples uses.  d_keys: (out1 - out0) uint64 scratch,
- * cleared here.  station_mask must be NULL.  Stream-ordered, no allocation,
- * no synchronisation. */
+ * cleared here.  station_mask must be NULL.  Stream-ordered; the traces are
+ * rearranged into stream-ordered scratch (cudaMallocAsync) where the table
+ * runs the tensor-memory kernel; no synchronisation. */
 BP_API int bp_record_beamform_max_dev(const bp_table *table, const bp_record *record,
                                       int storage, unsigned long long *d_keys,
                                       void *stream);
@@ -438,7 +439,11 @@ BP_API int bp_keys_from_shared_dev(const unsigned long long *d_keys, size_t n_sa
 /* ---- staged-kernel configurations (autotuning) -------------------------- */
 /* The staged kernel exists in several shapes (sources per thread, samples per
  * lane, consumer warps, ring stages, stations per ring stage, sources per
- * block, blocks per SM), all over the same 64-source tables.
+ * block, blocks per SM), all over the same 64-source tables.  The last config
+ * is the tensor-memory kernel, the built-in default of FP32 storage where a
+ * table's delay windows are narrow (bp_table_kernel_config tells); it takes
+ * stream-ordered scratch of about the traces' size (batches: for their
+ * lifetime), and the staged kernel runs where there is no memory for it.
  * bp_set_kernel_config chooses one per (storage, reduce) for every later
  * launch in the process (-1: built-in default); the environment variable
  * BEAMPOWER_B200_KERNEL_CONFIG overrides it.  beampower_b200/autotune.py
