@@ -152,7 +152,7 @@ __global__ void init_stats_kernel(int* stats, int* status) {
 
 template <int P>
 int launch_table_build(const int32_t* d, const float* w, bp::TableDev& tb, cudaStream_t st) {
-  const size_t smem = (size_t)(2 * tb.S * P + tb.S) * sizeof(int);
+  const size_t smem = (size_t)2 * tb.S * P * sizeof(int);
   if (smem > 48 * 1024)
     BP_CUDA(cudaFuncSetAttribute(bp::table_build_kernel<P>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -174,102 +174,69 @@ bool tiling_map_enabled() {
 
 // Source order for the tiles (see split_dim_kernel): d_perm[n_tiles * K],
 // original indices, -1 past the last source.  Segment boundaries depend only
-// on N and K (children split at a multiple of K); the data decide which
-// (station, phase) delay orders each segment.
+// on N and K; the data decide which (station, phase) delay orders each.
 int build_tiling_map(const int32_t* d_delays, const float* d_w, size_t N, size_t S, size_t P,
                      int K, int n_tiles, int* d_perm, cudaStream_t st) {
   const int total = n_tiles * K;
   bp::iota_perm_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_perm, (int)N, total);
   BP_LAUNCHED("iota_perm_kernel");
   if ((int)N <= K || !tiling_map_enabled()) return BP_OK;
-  // Host: per level, every segment in position order (begin, end, splitting?).
-  std::vector<int> seg_b, seg_e, seg_dim0, seg_of_tile;
-  std::vector<size_t> level_seg_off, level_tile_off;
-  std::vector<std::pair<int, int>> cur = {{0, (int)N}};
-  int max_segs = 1;
+  int levels = 0;  // of the whole grid, until one block takes a segment
   while (true) {
-    bool any_split = false;
-    for (auto& be : cur)
-      if (be.second - be.first > K) any_split = true;
-    if (!any_split) break;
-    level_seg_off.push_back(seg_b.size());
-    level_tile_off.push_back(seg_of_tile.size());
-    std::vector<std::pair<int, int>> next;
-    const int base = (int)seg_b.size();
-    for (size_t g = 0; g < cur.size(); ++g) {
-      const int b = cur[g].first, e = cur[g].second;
-      const bool split = e - b > K;
-      seg_b.push_back(b);
-      seg_e.push_back(e);
-      seg_dim0.push_back(split ? 0 : -1);
-      for (int t = b / K; t < (e + K - 1) / K; ++t) seg_of_tile.push_back((int)g);
-      if (split) {
-        const int left = ((e - b + K - 1) / K / 2) * K;
-        next.push_back({b, b + left});
-        next.push_back({b + left, e});
-      } else {
-        next.push_back({b, e});
-      }
+    int longest = 0;
+    for (int g = 0; g < (1 << levels); ++g) {
+      const int2 s = bp::map_segment((int)N, K, levels, g);
+      longest = std::max(longest, s.y - s.x);
     }
-    max_segs = std::max(max_segs, (int)seg_b.size() - base);
-    cur.swap(next);
+    if (longest <= bp::kMapBlock) break;
+    ++levels;
   }
-  if (level_seg_off.empty()) return BP_OK;
-  level_seg_off.push_back(seg_b.size());
-  level_tile_off.push_back(seg_of_tile.size());
-  int seg_bits = 1;
-  while ((1 << seg_bits) < max_segs) ++seg_bits;
-  size_t temp_bytes = 0;
-  {
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(
-        nullptr, temp_bytes, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
-        (const int*)nullptr, (int*)nullptr, (int)N, 0, 32 + seg_bits, st);
-    if (e != cudaSuccess) return cuda_fail(e, "radix sort size query");
-  }
-  const size_t ns = seg_b.size(), nt = seg_of_tile.size();
-  const size_t o_b = 0, o_e = o_b + pad256(ns * 4), o_d = o_e + pad256(ns * 4),
-               o_t = o_d + pad256(ns * 4), o_ka = o_t + pad256(nt * 4),
-               o_kb = o_ka + pad256(N * 8), o_pb = o_kb + pad256(N * 8),
-               o_tmp = o_pb + pad256(N * 4), bytes = o_tmp + pad256(temp_bytes);
   char* scratch = nullptr;
-  BP_CUDA(cudaMallocAsync(&scratch, bytes, st));
-  int* d_b = reinterpret_cast<int*>(scratch + o_b);
-  int* d_e = reinterpret_cast<int*>(scratch + o_e);
-  int* d_dim = reinterpret_cast<int*>(scratch + o_d);
-  int* d_tile = reinterpret_cast<int*>(scratch + o_t);
-  auto* d_ka = reinterpret_cast<unsigned long long*>(scratch + o_ka);
-  auto* d_kb = reinterpret_cast<unsigned long long*>(scratch + o_kb);
-  int* d_pb = reinterpret_cast<int*>(scratch + o_pb);
-  cudaError_t e = cudaMemcpyAsync(d_b, seg_b.data(), ns * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_e, seg_e.data(), ns * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_dim, seg_dim0.data(), ns * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_tile, seg_of_tile.data(), nt * 4, cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaSuccess;
   int* p_cur = d_perm;
-  int* p_next = d_pb;
-  for (size_t L = 0; e == cudaSuccess && L + 1 < level_seg_off.size(); ++L) {
-    const int nseg = (int)(level_seg_off[L + 1] - level_seg_off[L]);
-    int* ldim = d_dim + level_seg_off[L];
-    bp::split_dim_kernel<<<nseg, 128, 0, st>>>(d_delays, d_w, (int)S, (int)P, p_cur,
-                                               d_b + level_seg_off[L], d_e + level_seg_off[L],
-                                               ldim);
-    bp::split_keys_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(
-        d_delays, (int)(S * P), (int)N, K, p_cur, d_tile + level_tile_off[L], ldim, d_ka);
-    g_launches.fetch_add(2, std::memory_order_relaxed);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) {
-      size_t tb = temp_bytes;
-      e = cub::DeviceRadixSort::SortPairs(scratch + o_tmp, tb, d_ka, d_kb, p_cur, p_next, (int)N,
-                                          0, 32 + seg_bits, st);
+  if (levels > 0) {
+    size_t temp_bytes = 0;
+    e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, (const unsigned long long*)nullptr,
+                                        (unsigned long long*)nullptr, (const int*)nullptr,
+                                        (int*)nullptr, (int)N, 0, 32 + levels, st);
+    if (e != cudaSuccess) return cuda_fail(e, "radix sort size query");
+    const size_t o_d = 0, o_ka = o_d + pad256(sizeof(int) << levels),
+                 o_kb = o_ka + pad256(N * 8), o_pb = o_kb + pad256(N * 8),
+                 o_tmp = o_pb + pad256(N * 4), bytes = o_tmp + pad256(temp_bytes);
+    BP_CUDA(cudaMallocAsync(&scratch, bytes, st));
+    int* d_dim = reinterpret_cast<int*>(scratch + o_d);
+    auto* d_ka = reinterpret_cast<unsigned long long*>(scratch + o_ka);
+    auto* d_kb = reinterpret_cast<unsigned long long*>(scratch + o_kb);
+    int* p_next = reinterpret_cast<int*>(scratch + o_pb);
+    for (int L = 0; e == cudaSuccess && L < levels; ++L) {
+      bp::split_dim_kernel<<<1u << L, 512, 0, st>>>(d_delays, d_w, (int)S, (int)P, (int)N, K, L,
+                                                     p_cur, d_dim);
+      bp::split_keys_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(
+          d_delays, (int)(S * P), (int)N, K, L, p_cur, d_dim, d_ka);
+      g_launches.fetch_add(2, std::memory_order_relaxed);
+      e = cudaGetLastError();
+      if (e == cudaSuccess) {
+        size_t tb = temp_bytes;
+        e = cub::DeviceRadixSort::SortPairs(scratch + o_tmp, tb, d_ka, d_kb, p_cur, p_next,
+                                            (int)N, 0, 32 + L, st);
+      }
+      std::swap(p_cur, p_next);
     }
-    std::swap(p_cur, p_next);
+    if (e == cudaSuccess && p_cur != d_perm)
+      e = cudaMemcpyAsync(d_perm, p_cur, N * 4, cudaMemcpyDeviceToDevice, st);
   }
-  if (e == cudaSuccess && p_cur != d_perm)
-    e = cudaMemcpyAsync(d_perm, p_cur, N * 4, cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(bp::split_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(bp::MapBlock));
+  if (e == cudaSuccess) {
+    bp::split_block_kernel<<<1u << levels, 1024, sizeof(bp::MapBlock), st>>>(
+        d_delays, d_w, (int)S, (int)P, (int)N, K, levels, d_perm);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    e = cudaGetLastError();
+  }
   int rc = BP_OK;
   if (e != cudaSuccess) rc = cuda_fail(e, "tiling map");
-  cudaFreeAsync(scratch, st);
+  if (scratch) cudaFreeAsync(scratch, st);
   return rc;
 }
 
@@ -807,7 +774,8 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
   };
   init_stats_kernel<<<1, 32, 0, st>>>(t->dev.stats, t->status);
   g_launches.fetch_add(1);
-  if (N > 0) {
+  t->dev.minmax = t->minmax;
+  if (N > 0 && !window) {  // else written by the table build
     bp::minmax_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(d_delays, d_weights, (int)N,
                                                                   (int)S, (int)P, t->minmax);
     g_launches.fetch_add(1);

@@ -62,6 +62,7 @@ struct TableDev {
   int* st_spread;    // [n_tiles * S * P] window span beyond the time tile
   void* meta;        // [n_tiles * S * K] MetaT<P>
   int* stats;        // [kStatCount]
+  int* minmax;       // (N, 2) per source, source order
   const int* perm;   // optional [n_tiles * K] source order (nullptr: identity)
   int index_base;    // added to every source index (a table over part of a grid)
 };
@@ -103,7 +104,7 @@ __host__ __device__ __forceinline__ int floor_align(int v) {
 
 // ---------------------------------------------------------------------------
 // Table build: one block per source tile.
-// Dynamic shared memory: 2 * S * P ints (per-station lo / hi) + S ints.
+// Dynamic shared memory: 2 * S * P ints (per-station lo / hi).
 // ---------------------------------------------------------------------------
 template <int P>
 __global__ void table_build_kernel(const int32_t* __restrict__ delays,
@@ -113,7 +114,6 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
   const int S = tb.S, K = tb.K;
   int* lo = sh;               // [S * P]
   int* hi = lo + S * P;       // [S * P]
-  int* slot = hi + S * P;     // [S] active slot of station s, or -1
   __shared__ int n_active_sh;
   const int tile = blockIdx.x;
 
@@ -123,88 +123,103 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
     return (o >= 0 && o < tb.N) ? o : -1;
   };
 
-  // 1. per source: min / max over weighted stations, non-finite weights.
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
+  // 1. A warp per source, lanes over its (station, phase) entries: the source's
+  // min / max over weighted stations, the tile's windows, the kinds of weights.
+  // (A thread per source and then one per window read every row twice, the
+  // first time uncoalesced: 420 us on the 400,000-source grid.)
+  const int D = S * P, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_warps = blockDim.x >> 5;
+  for (int sp = threadIdx.x; sp < D; sp += blockDim.x) {
+    lo[sp] = INT_MAX;
+    hi[sp] = INT_MIN;
+  }
+  __syncthreads();
+  int bad = 0, real = 0;
+  for (int k = warp; k < K; k += n_warps) {
     const int o = orig_of(k);
-    int mn = INT_MAX, mx = INT_MIN, bad = 0, real = 0;
+    int mn = INT_MAX, mx = INT_MIN;
     if (o >= 0) {
-      const int32_t* d = delays + (size_t)o * S * P;
+      const int32_t* d = delays + (size_t)o * D;
       const float* w = weights + (size_t)o * S;
-      for (int s = 0; s < S; ++s) {
-        const float ws = w[s];
+#pragma unroll 4
+      for (int sp = lane; sp < D; sp += 32) {
+        const float ws = w[sp / P];
+        const int v = d[sp];
         if (ws == 0.0f) continue;
         if (!isfinite(ws)) bad = 1;
         real |= ws != 1.0f;
-        for (int p = 0; p < P; ++p) {
-          const int v = d[s * P + p];
-          mn = min(mn, v);
-          mx = max(mx, v);
-        }
+        mn = min(mn, v);
+        mx = max(mx, v);
+        atomicMin(&lo[sp], v);
+        atomicMax(&hi[sp], v);
+      }
+      mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+      mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    }
+    if (lane == 0) {
+      tb.src_info[(size_t)tile * K + k] = make_int4(o >= 0 ? o + tb.index_base : o, mn, mx, 0);
+      if (o >= 0) {
+        tb.minmax[2 * (size_t)o] = mn;
+        tb.minmax[2 * (size_t)o + 1] = mx;
       }
     }
-    tb.src_info[(size_t)tile * K + k] = make_int4(o >= 0 ? o + tb.index_base : o, mn, mx, 0);
-    if (bad) atomicOr(&tb.stats[kStatNonFinite], 1);
-    if (real) atomicOr(&tb.stats[kStatReal], 1);
   }
-  // 2. per (station, phase): window over the tile's weighted sources.
-  for (int sp = threadIdx.x; sp < S * P; sp += blockDim.x) {
-    const int s = sp / P;
-    int l = INT_MAX, h = INT_MIN;
-    for (int k = 0; k < K; ++k) {
-      const int o = orig_of(k);
-      if (o < 0) continue;
-      if (weights[(size_t)o * S + s] == 0.0f) continue;
-      const int v = delays[(size_t)o * S * P + sp];
-      l = min(l, v);
-      h = max(h, v);
-    }
-    lo[sp] = l;
-    hi[sp] = h;
-  }
+  if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(&tb.stats[kStatNonFinite], 1);
+  if (__any_sync(0xFFFFFFFFu, real) && lane == 0) atomicOr(&tb.stats[kStatReal], 1);
   __syncthreads();
-  // 3. active station list, ascending station index (the summation order).
-  if (threadIdx.x == 0) {
+  // 2. One warp: the active stations in ascending order (the summation order),
+  // their windows, the statistics.
+  if (warp == 0) {
     unsigned long long spread_sum = 0;
     int n = 0, spread_max = 0, mn = INT_MAX, mx = INT_MIN, lo_al_min = INT_MAX, wide = 0;
-    for (int s = 0; s < S; ++s) {
-      if (lo[s * P] > hi[s * P]) {  // no weighted source in this tile
-        slot[s] = -1;
-        continue;
+    for (int s0 = 0; s0 < S; s0 += 32) {
+      const int s = s0 + lane;
+      const bool used = s < S && lo[s * P] <= hi[s * P];  // a weighted source in this tile
+      const unsigned bal = __ballot_sync(0xFFFFFFFFu, used);
+      if (used) {
+        const int j = n + __popc(bal & ((1u << lane) - 1u));
+        tb.st_s[(size_t)tile * S + j] = s;
+        for (int p = 0; p < P; ++p) {
+          const int l = lo[s * P + p], h = hi[s * P + p];
+          const int la = floor_align(l);
+          const long long span = (long long)h - la;
+          if (span > 0xFFFF) wide = 1;
+          const int sp32 = (int)min(span, (long long)INT_MAX);
+          tb.st_lo[((size_t)tile * S + j) * P + p] = la;
+          tb.st_spread[((size_t)tile * S + j) * P + p] = sp32;
+          spread_max = max(spread_max, sp32);
+          spread_sum += (unsigned long long)sp32;
+          mn = min(mn, l);
+          mx = max(mx, h);
+          lo_al_min = min(lo_al_min, la);
+        }
       }
-      slot[s] = n;
-      tb.st_s[(size_t)tile * S + n] = s;
-      for (int p = 0; p < P; ++p) {
-        const int l = lo[s * P + p], h = hi[s * P + p];
-        const int la = floor_align(l);
-        const long long span = (long long)h - la;
-        if (span > 0xFFFF) wide = 1;
-        const int sp32 = (int)min(span, (long long)INT_MAX);
-        tb.st_lo[((size_t)tile * S + n) * P + p] = la;
-        tb.st_spread[((size_t)tile * S + n) * P + p] = sp32;
-        spread_max = max(spread_max, sp32);
-        spread_sum += (unsigned long long)sp32;
-        mn = min(mn, l);
-        mx = max(mx, h);
-        lo_al_min = min(lo_al_min, la);
+      n += __popc(bal);
+    }
+    spread_max = __reduce_max_sync(0xFFFFFFFFu, spread_max);
+    mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    lo_al_min = __reduce_min_sync(0xFFFFFFFFu, lo_al_min);
+    wide = __any_sync(0xFFFFFFFFu, wide);
+    for (int o = 16; o > 0; o >>= 1) spread_sum += __shfl_xor_sync(0xFFFFFFFFu, spread_sum, o);
+    if (lane == 0) {
+      n_active_sh = n;
+      tb.tile_hdr[tile] = make_int2(n, 0);
+      if (n > 0) {
+        atomicMin(&tb.stats[kStatMinDelay], mn);
+        atomicMax(&tb.stats[kStatMaxDelay], mx);
+        atomicMin(&tb.stats[kStatMinLoAligned], lo_al_min);
       }
-      ++n;
+      atomicMax(&tb.stats[kStatMaxSpread], spread_max);
+      atomicMax(&tb.stats[kStatMaxActive], n);
+      auto* sums = reinterpret_cast<unsigned long long*>(tb.stats);
+      atomicAdd(&sums[kStatSpreadRows / 2], (unsigned long long)(n * P));
+      atomicAdd(&sums[kStatSpreadSum / 2], spread_sum);
+      if (wide) atomicOr(&tb.stats[kStatWideTile], 1);
     }
-    n_active_sh = n;
-    tb.tile_hdr[tile] = make_int2(n, 0);
-    if (n > 0) {
-      atomicMin(&tb.stats[kStatMinDelay], mn);
-      atomicMax(&tb.stats[kStatMaxDelay], mx);
-      atomicMin(&tb.stats[kStatMinLoAligned], lo_al_min);
-    }
-    atomicMax(&tb.stats[kStatMaxSpread], spread_max);
-    atomicMax(&tb.stats[kStatMaxActive], n);
-    auto* sums = reinterpret_cast<unsigned long long*>(tb.stats);
-    atomicAdd(&sums[kStatSpreadRows / 2], (unsigned long long)(n * P));
-    atomicAdd(&sums[kStatSpreadSum / 2], spread_sum);
-    if (wide) atomicOr(&tb.stats[kStatWideTile], 1);
   }
   __syncthreads();
-  // 4. per (active station, source): weight and 16-bit offsets.
+  // 3. per (active station, source): weight and 16-bit offsets.
   const int n_active = n_active_sh;
   M* meta = reinterpret_cast<M*>(tb.meta) + (size_t)tile * S * K;
   for (int idx = threadIdx.x; idx < n_active * K; idx += blockDim.x) {
@@ -1439,86 +1454,385 @@ __global__ void differential_kernel(const float* __restrict__ traces, long long 
 // Source tiling map: recursive median splits of the sources on their delay
 // vectors (a k-d tree over the (station, phase) delays), so that the 64
 // sources of a tile are close in delay space and every station's delay
-// window inside a tile is short.  Each level: pick per splitting segment the
+// window inside a tile is short.  Each split orders a segment's sources by the
 // (station, phase) whose weighted delays vary most (variance over up to 256
-// evenly spaced members), then one global stable radix sort of all sources
-// on (segment, delay) keys orders every splitting segment by that delay and
-// leaves finished segments in place; children split at a multiple of the
-// tile size.  Only the grouping changes: keys and outputs use the original
-// source index.
+// evenly spaced members) and cuts it at a multiple of the tile size.  Segments
+// longer than kMapBlock sources are split level by level over the whole grid
+// (one radix sort on (segment, delay) keys per level); then one block per
+// segment makes all of its further splits in shared memory.  Only the grouping
+// changes: keys and outputs use the original source index.
+// (With a level for every split and one thread per (station, phase) in the
+// choice of the split, which waits for its 256 members one after the other, a
+// whole table build took 1.17 ms for 4,000 sources x 20 stations and 5.8 ms for
+// 400,000 x 60; it takes 0.28 and 1.8 ms.)
 // ---------------------------------------------------------------------------
-__global__ void split_dim_kernel(const int32_t* __restrict__ delays,
-                                 const float* __restrict__ weights, int S, int P,
-                                 const int* __restrict__ perm, const int* __restrict__ seg_begin,
-                                 const int* __restrict__ seg_end, int* __restrict__ seg_dim) {
-  const int g = blockIdx.x;
-  const int b = seg_begin[g], e = seg_end[g];
-  const int len = e - b;
-  const int D = S * P;
-  if (len <= 0 || seg_dim[g] < 0) return;  // finished segment (dim preset to -1)
-  const int n_sample = min(len, 256);
-  __shared__ double best_v[32];
-  __shared__ int best_d[32];
-  double bv = -1.0;
-  int bd = 0;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    const int s = d / P;
-    double sum = 0.0, sq = 0.0;
-    int n = 0;
-    for (int j = 0; j < n_sample; ++j) {
-      const int o = perm[b + (int)(((long long)len * j) / n_sample)];
-      if (weights[(size_t)o * S + s] == 0.0f) continue;
-      const double v = (double)delays[(size_t)o * D + d];
-      sum += v;
-      sq += v * v;
-      ++n;
-    }
-    const double var = n > 1 ? (sq - sum * sum / n) / n : 0.0;
-    if (var > bv) {  // ascending d per thread: the lower d wins ties
-      bv = var;
-      bd = d;
-    }
+constexpr int kMapBlock = 4096;
+constexpr int kMapSample = 256;  // members a split looks at, at most
+constexpr int kMapDims = 128;    // (station, phase) pairs it looks at together
+
+// Members of the left part of a segment of len sources.
+__host__ __device__ inline int map_left(int len, int K) { return (len + K - 1) / K / 2 * K; }
+
+// Segment g of level L ([0, N) is level 0): every segment is split on the
+// way down.
+__host__ __device__ inline int2 map_segment(int N, int K, int level, int g) {
+  int b = 0, e = N;
+  for (int bit = level - 1; bit >= 0; --bit) {
+    const int left = map_left(e - b, K);
+    if ((g >> bit) & 1) b += left;
+    else e = b + left;
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ov = __shfl_down_sync(0xFFFFFFFFu, bv, off);
-    const int od = __shfl_down_sync(0xFFFFFFFFu, bd, off);
-    if (ov > bv || (ov == bv && od < bd)) {
-      bv = ov;
-      bd = od;
-    }
-  }
-  if ((threadIdx.x & 31) == 0) {
-    best_v[threadIdx.x >> 5] = bv;
-    best_d[threadIdx.x >> 5] = bd;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double v = -1.0;
-    int d = 0;
-    for (int w = 0; w < (int)((blockDim.x + 31) / 32); ++w)
-      if (best_v[w] > v || (best_v[w] == v && best_d[w] < d)) {
-        v = best_v[w];
-        d = best_d[w];
-      }
-    seg_dim[g] = d;
-  }
+  return make_int2(b, e);
 }
 
-// Composite sort key of every source position for one level:
-// (segment index << 32) | biased delay on the segment's split dimension
-// (0 for finished segments, which therefore keep their order).
+// A warp's sums over its members: per (station, phase) the number of weighted
+// members, their delays (from the first member's) and the squares.  FP32: they
+// only choose the split.  (Double sums added by shared-memory atomics took 40
+// us per split.)
+struct MapSums {
+  float n[kMapDims], sum[kMapDims], sq[kMapDims];
+};
+
+// The (station, phase) whose weighted delays vary most over members b .. e - 1
+// (member(i): a source index), by `nw` warps (this thread's is warp `w` of
+// them), the lowest one among equals.  Lanes take four (station, phase) pairs
+// each, warps every nw-th member.  part: a MapSums per warp of the group; sync:
+// a barrier of its warps.
+template <class Member, class Sync>
+__device__ int map_widest(const int32_t* __restrict__ delays, const float* __restrict__ weights,
+                          int S, int P, Member member, int b, int e, int w, int nw,
+                          MapSums* part, int* best_dim, Sync sync) {
+  const int lane = threadIdx.x & 31, D = S * P, len = e - b;
+  const int n_sample = min(len, kMapSample);
+  // member j of kMapSample evenly spaced ones, or of all
+  auto pick = [&](int j) {
+    return (size_t)member(b + (len <= kMapSample ? j
+                                                 : (int)((long long)len * j / kMapSample)));
+  };
+  float bv = -1.0f;
+  int bd = 0;
+  const size_t o0 = (size_t)member(b) * D;
+  for (int d0 = 0; d0 < D; d0 += kMapDims) {
+    float n[4] = {}, a[4] = {}, q[4] = {};
+    int from[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) from[x] = delays[o0 + min(d0 + 32 * x + lane, D - 1)];
+    int dim[4], sta[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      dim[x] = min(d0 + 32 * x + lane, D - 1);
+      sta[x] = dim[x] / P;
+    }
+    auto add = [&](auto nx) {  // nx: 32-wide columns in use
+#pragma unroll 4
+      for (int j = w; j < n_sample; j += nw) {
+        const size_t o = pick(j);
+#pragma unroll
+        for (int x = 0; x < decltype(nx)::value; ++x) {
+          const float v = (float)delays[o * D + dim[x]] - (float)from[x];
+          const float used = weights[o * S + sta[x]] == 0.0f ? 0.0f : 1.0f;
+          n[x] += used;
+          a[x] += used * v;
+          q[x] += used * v * v;
+        }
+      }
+    };
+    if (D - d0 <= 32) add(std::integral_constant<int, 1>{});
+    else if (D - d0 <= 64) add(std::integral_constant<int, 2>{});
+    else add(std::integral_constant<int, 4>{});
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      part[w].n[32 * x + lane] = n[x];
+      part[w].sum[32 * x + lane] = a[x];
+      part[w].sq[32 * x + lane] = q[x];
+    }
+    sync();
+    if (w == 0) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = 32 * x + lane;
+        if (d0 + i >= D) continue;
+        float c = n[x], t = a[x], u = q[x];
+        for (int v = 1; v < nw; ++v) {
+          c += part[v].n[i];
+          t += part[v].sum[i];
+          u += part[v].sq[i];
+        }
+        const float var = c > 1.0f ? (u - t * t / c) / c : 0.0f;
+        if (var > bv) {
+          bv = var;
+          bd = d0 + i;
+        }
+      }
+    }
+    sync();
+  }
+  if (w == 0) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_down_sync(0xFFFFFFFFu, bv, o);
+      const int od = __shfl_down_sync(0xFFFFFFFFu, bd, o);
+      if (ov > bv || (ov == bv && od < bd)) {
+        bv = ov;
+        bd = od;
+      }
+    }
+    if (lane == 0) *best_dim = bd;
+  }
+  sync();
+  return *best_dim;
+}
+
+// One level over the whole grid: block g chooses segment g's split ...
+__global__ void __launch_bounds__(512)
+split_dim_kernel(const int32_t* __restrict__ delays, const float* __restrict__ weights, int S,
+                 int P, int N, int K, int level, const int* __restrict__ perm,
+                 int* __restrict__ seg_dim) {
+  __shared__ MapSums part[16];
+  __shared__ int best;
+  const int2 seg = map_segment(N, K, level, blockIdx.x);
+  const int d = map_widest(
+      delays, weights, S, P, [&](int i) { return perm[i]; }, seg.x, seg.y, threadIdx.x >> 5,
+      blockDim.x >> 5, part, &best, [] { __syncthreads(); });
+  if (threadIdx.x == 0) seg_dim[blockIdx.x] = d;
+}
+
+// ... and every source position gets its sort key (segment << 32) | biased
+// delay on the segment's split dimension.
 __global__ void split_keys_kernel(const int32_t* __restrict__ delays, int D, int N, int K,
-                                  const int* __restrict__ perm,
-                                  const int* __restrict__ seg_of_tile,
+                                  int level, const int* __restrict__ perm,
                                   const int* __restrict__ seg_dim,
                                   unsigned long long* __restrict__ keys) {
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= N) return;
-  const int g = seg_of_tile[pos / K];
-  const int d = seg_dim[g];
-  uint32_t low = 0u;
-  if (d >= 0) low = (uint32_t)delays[(size_t)perm[pos] * D + d] ^ 0x80000000u;
+  int b = 0, e = N, g = 0;
+  for (int l = 0; l < level; ++l) {
+    const int left = map_left(e - b, K);
+    if (pos >= b + left) {
+      b += left;
+      g = 2 * g + 1;
+    } else {
+      e = b + left;
+      g = 2 * g;
+    }
+  }
+  const uint32_t low = (uint32_t)delays[(size_t)perm[pos] * D + seg_dim[g]] ^ 0x80000000u;
   keys[pos] = ((unsigned long long)(uint32_t)g << 32) | low;
+}
+
+// Shared memory of split_block_kernel.
+constexpr int kMapParts = kMapBlock / kTableTile;
+struct MapBlock {
+  int idx[2][kMapBlock];
+  MapSums part[32];
+  int best[32];
+  int cut[kMapParts + 2], dim[kMapParts + 1];
+  uint32_t value[kMapParts + 1];  // the left part's largest delay (biased)
+  int below[kMapParts + 1];       // members smaller than it
+  int count[2][kMapParts + 1];
+  int at_cut[kMapParts + 1];
+  int warp_sum[32];
+  int n_cut;
+};
+
+// All splits below one segment of a level (at most kMapBlock sources), one
+// block of 1024 threads per segment, four places per thread (a warp has 128
+// consecutive ones, as four rows).  Per level: the splits of its parts (warps in
+// groups, a group per part), the delay at which each part is cut (selected bit
+// by bit, all parts together), then a stable partition around it.  What bounds
+// it is the chain of barriers, and on many stations the latency of the members
+// that the splits read: 220 us for 4,000 x 20 (six levels), 490 us for 400,000 x
+// 60 (128 segments).  (A bitonic sort of (part, delay) keys has 78 barriers per
+// level where the selection has two per delay bit that differs, about ten: 500
+// us and 750 us.)
+__global__ void __launch_bounds__(1024)
+split_block_kernel(const int32_t* __restrict__ delays, const float* __restrict__ weights, int S,
+                   int P, int N, int K, int level, int* __restrict__ perm) {
+  extern __shared__ __align__(16) unsigned char map_smem[];
+  MapBlock& m = *reinterpret_cast<MapBlock*>(map_smem);
+  constexpr int ROWS = kMapBlock / 1024;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = S * P;
+  const unsigned before = (1u << lane) - 1u;
+  const int2 seg = map_segment(N, K, level, blockIdx.x);
+  const int n = seg.y - seg.x;
+  for (int i = tid; i < n; i += blockDim.x) m.idx[0][i] = perm[seg.x + i];
+  if (tid == 0) {
+    m.cut[0] = 0;
+    m.cut[1] = n;
+    m.n_cut = 1;
+  }
+  __syncthreads();
+  int cur = 0;
+  // Places before this thread's places whose flag is set (flag[r]: of its place
+  // in row r); every thread calls it.
+  auto places_before = [&](const bool (&flag)[ROWS], int (&out)[ROWS]) {
+    int sum = 0;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const unsigned f = __ballot_sync(0xFFFFFFFFu, flag[r]);
+      out[r] = sum + __popc(f & before);
+      sum += __popc(f);
+    }
+    if (lane == 0) m.warp_sum[warp] = sum;
+    __syncthreads();
+    int from = lane < warp ? m.warp_sum[lane] : 0;
+    from = __reduce_add_sync(0xFFFFFFFFu, from);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) out[r] += from;
+    __syncthreads();
+  };
+  while (true) {
+    const int parts = m.n_cut;
+    bool any = false;
+    for (int g = 0; g < parts; ++g) any |= m.cut[g + 1] - m.cut[g] > K;
+    if (!any) break;
+    // groups of nw warps (a power of two; not 2: barrier 0 is the block's, and
+    // 15 others are too few for 16 groups)
+    int nw = 32;
+    while (nw > 1 && 32 / nw < parts) nw /= 2;
+    if (nw == 2) nw = 1;
+    const int groups = 32 / nw, grp = warp / nw;
+    for (int g = grp; g < parts; g += groups) {
+      const int b = m.cut[g], e = m.cut[g + 1];
+      if (e - b <= K) continue;
+      const int* idx = m.idx[cur];
+      auto member = [&](int i) { return idx[i]; };
+      const int d = map_widest(delays, weights, S, P, member, b, e, warp - grp * nw, nw,
+                               m.part + grp * nw, &m.best[grp], [&] {
+                                 if (nw == 1) __syncwarp();
+                                 else named_barrier_sync(1 + grp, nw * 32);
+                               });
+      if (warp == grp * nw && lane == 0) m.dim[g] = d;
+    }
+    if (tid < parts) {
+      m.value[tid] = 0u;
+      m.below[tid] = 0;
+      m.count[0][tid] = m.count[1][tid] = 0;
+    }
+    __syncthreads();
+    // Each place's part (parts past the end: a split of nothing) and delay.
+    int part[ROWS], source[ROWS];
+    uint32_t u[ROWS];
+    unsigned peers[ROWS];  // this row's lanes in the same part
+    uint32_t any_set = 0u, all_set = 0xFFFFFFFFu;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int i = warp * 32 * ROWS + r * 32 + lane;
+      int g = -1;
+      if (i < n) {
+        g = 0;  // cut[g] <= i < cut[g + 1]
+        for (int h = parts; h - g > 1;) {
+          const int mid = (g + h) >> 1;
+          if (m.cut[mid] <= i) g = mid;
+          else h = mid;
+        }
+      }
+      const bool split = g >= 0 && m.cut[g + 1] - m.cut[g] > K;
+      part[r] = split ? g : -1;
+      source[r] = i < n ? m.idx[cur][i] : 0;
+      u[r] = 0u;
+      if (split) {
+        u[r] = (uint32_t)delays[(size_t)source[r] * D + m.dim[g]] ^ 0x80000000u;
+        any_set |= u[r];
+        all_set &= u[r];
+      }
+      peers[r] = __match_any_sync(0xFFFFFFFFu, part[r]);
+    }
+    // The bits that differ between any two delays: those above are common.
+    any_set = __reduce_or_sync(0xFFFFFFFFu, any_set);
+    all_set = __reduce_and_sync(0xFFFFFFFFu, all_set);
+    if (lane == 0) {
+      m.best[warp] = (int)any_set;
+      m.warp_sum[warp] = (int)all_set;
+    }
+    __syncthreads();
+    any_set = __reduce_or_sync(0xFFFFFFFFu, (unsigned)m.best[lane]);
+    all_set = __reduce_and_sync(0xFFFFFFFFu, (unsigned)m.warp_sum[lane]);
+    __syncthreads();
+    const uint32_t differ = any_set ^ all_set;
+    const int bits = 32 - __clz((int)differ);
+    const uint32_t common = bits < 32 ? any_set >> bits << bits : 0u;
+    // value[g]: the largest v with fewer than left + 1 members below it, so the
+    // delay of the member that is `left`-th from the smallest.
+    for (int bit = bits - 1; bit >= 0; --bit) {
+      int* count = m.count[bit & 1];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const uint32_t v = (part[r] >= 0 ? (m.value[part[r]] | common) : 0u) | (1u << bit);
+        const unsigned less = __ballot_sync(0xFFFFFFFFu, part[r] >= 0 && u[r] < v);
+        if (part[r] >= 0 && (peers[r] & before) == 0u && (less & peers[r]) != 0u)
+          atomicAdd(&count[part[r]], __popc(less & peers[r]));
+      }
+      __syncthreads();
+      if (tid < parts) {
+        const int len = m.cut[tid + 1] - m.cut[tid];
+        if (len > K && count[tid] <= map_left(len, K)) {
+          m.value[tid] |= 1u << bit;
+          m.below[tid] = count[tid];
+        }
+        m.count[(bit & 1) ^ 1][tid] = 0;
+      }
+      __syncthreads();
+    }
+    // Left: the members below the cut's delay, and of those at it the first
+    // ones, as many as the left part still takes.
+    bool flag[ROWS];
+    int rank[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+      flag[r] = part[r] >= 0 && u[r] == (m.value[part[r]] | common);
+    places_before(flag, rank);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int i = warp * 32 * ROWS + r * 32 + lane;
+      if (part[r] >= 0 && i == m.cut[part[r]]) m.at_cut[part[r]] = rank[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      if (part[r] < 0) {
+        flag[r] = false;
+        continue;
+      }
+      const int g = part[r], left = map_left(m.cut[g + 1] - m.cut[g], K);
+      flag[r] = flag[r] ? rank[r] - m.at_cut[g] < left - m.below[g]
+                        : u[r] < (m.value[g] | common);
+    }
+    places_before(flag, rank);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int i = warp * 32 * ROWS + r * 32 + lane;
+      if (part[r] >= 0 && i == m.cut[part[r]]) m.at_cut[part[r]] = rank[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int i = warp * 32 * ROWS + r * 32 + lane;
+      int to = i;
+      if (part[r] >= 0) {
+        const int b = m.cut[part[r]], lefts = rank[r] - m.at_cut[part[r]];
+        to = flag[r] ? b + lefts
+                     : b + map_left(m.cut[part[r] + 1] - b, K) + (i - b) - lefts;
+      }
+      if (i < n) m.idx[cur ^ 1][to] = source[r];
+    }
+    __syncthreads();
+    if (tid == 0) {  // the parts of the next level, from the last one
+      int next = 0;
+      for (int g = 0; g < parts; ++g) next += m.cut[g + 1] - m.cut[g] > K ? 2 : 1;
+      int at = next, end = n;
+      m.cut[at] = n;
+      for (int g = parts - 1; g >= 0; --g) {
+        const int b = m.cut[g], len = end - b;
+        end = b;
+        if (len > K) m.cut[--at] = b + map_left(len, K);
+        m.cut[--at] = b;
+      }
+      m.n_cut = next;
+    }
+    cur ^= 1;
+    __syncthreads();
+  }
+  for (int i = tid; i < n; i += blockDim.x) perm[seg.x + i] = m.idx[cur][i];
 }
 
 __global__ void iota_perm_kernel(int* __restrict__ perm, int N, int total) {
