@@ -6,21 +6,21 @@
 //
 // Exactness rests on three restatements:
 //  * NumPy's float32 sum (inside mean and std) is a pairwise sum whose split
-//    points depend on the length only.  The split tree is built on the host;
-//    its leaves are summed in parallel and its inner nodes level by level,
+//    points depend on the length only, so every node is found from its path
+//    from the root.  Leaves are summed in parallel, and nodes level by level,
 //    each with the same rounded operations as NumPy's loop.
 //  * NumPy's median is an order statistic (the mean of the two middle values
-//    for even lengths); a 4-pass 8-bit radix select on the order-preserving
-//    integer image of the floats finds it exactly.
+//    for even lengths); a radix select on the order-preserving integer image of
+//    the floats finds it exactly.
 //  * SciPy's distance rule is a greedy pass in decreasing height.  Its result
 //    is also the fixed point of rounds in which every undecided peak with no
 //    higher undecided peak within the distance is kept, and then every
 //    undecided peak within the distance of a kept one is dropped.
 #define BP_TEMPLATE_KERNELS_ONLY
 #include <cmath>
-#include <map>
-#include <mutex>
 #include <utility>
+
+#include <cooperative_groups.h>
 
 #include "bp_stats.cuh"
 
@@ -34,249 +34,342 @@ namespace {
 // The reduction then adds that sum to its initial +0.0.
 constexpr int kPwLeaf = 128;
 
-__host__ __device__ inline float add_rn(float a, float b) {
-#ifdef __CUDA_ARCH__
-  return __fadd_rn(a, b);
-#else
-  return a + b;
-#endif
-}
+__host__ __device__ inline int pw_left(int len) { return len / 2 - len / 2 % 8; }
 
-template <class Get>
-__host__ __device__ inline float pw_leaf(const Get& get, int len) {
+float pw_host(const float* x, int len) {
   if (len < 8) {
     float r = 0.0f;
-    for (int i = 0; i < len; ++i) r = add_rn(r, get(i));
+    for (int i = 0; i < len; ++i) r += x[i];
     return r;
   }
-  float r0 = get(0), r1 = get(1), r2 = get(2), r3 = get(3);
-  float r4 = get(4), r5 = get(5), r6 = get(6), r7 = get(7);
-  int i = 8;
-  const int lim = len - len % 8;
-  for (; i < lim; i += 8) {
-    r0 = add_rn(r0, get(i + 0));
-    r1 = add_rn(r1, get(i + 1));
-    r2 = add_rn(r2, get(i + 2));
-    r3 = add_rn(r3, get(i + 3));
-    r4 = add_rn(r4, get(i + 4));
-    r5 = add_rn(r5, get(i + 5));
-    r6 = add_rn(r6, get(i + 6));
-    r7 = add_rn(r7, get(i + 7));
+  if (len > kPwLeaf) {
+    const int n2 = pw_left(len);
+    return pw_host(x, n2) + pw_host(x + n2, len - n2);
   }
-  float res = add_rn(add_rn(add_rn(r0, r1), add_rn(r2, r3)), add_rn(add_rn(r4, r5), add_rn(r6, r7)));
-  for (; i < len; ++i) res = add_rn(res, get(i));
+  float r[8];
+  for (int k = 0; k < 8; ++k) r[k] = x[k];
+  int i = 8;
+  for (; i < len - len % 8; i += 8)
+    for (int k = 0; k < 8; ++k) r[k] += x[i + k];
+  float res = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
+  for (; i < len; ++i) res += x[i];
   return res;
 }
 
-// The split tree of a length: leaves {node, begin, len}, inner nodes
-// {node, left, right} grouped by height (children always lower).
-struct PwTree {
-  std::vector<int4> leaves;
-  std::vector<int4> inner;
-  std::vector<int> level_end;
-  int n_nodes = 0;
-  int root = 0;
+// Depth of the deepest leaf (the right child is the longer one).
+int pw_depth(int len) {
+  int d = 0;
+  for (; len > kPwLeaf; ++d) len -= pw_left(len);
+  return d;
+}
+
+// The node at the end of a path of `bits` turns (the highest bit first; 1:
+// right) from a node.  A path that goes on below a leaf is the leaf's when the
+// rest of it turns left, else nothing's (len 0).
+struct PwNode {
+  int begin, len;
+  __device__ PwNode down(int path, int bits) const {
+    PwNode v = *this;
+    for (int b = bits - 1; b >= 0; --b) {
+      const bool right = (path >> b) & 1, leaf = v.len <= kPwLeaf;
+      const int n2 = (int)((unsigned)v.len >> 1 & ~7u);  // pw_left
+      v.begin += right && !leaf ? n2 : 0;
+      v.len = leaf ? (right ? 0 : v.len) : right ? v.len - n2 : n2;
+    }
+    return v;
+  }
 };
 
-int pw_build(int begin, int len, std::vector<int4>& leaves, std::vector<int4>& inner,
-             std::vector<int>& height, int& next_id, int* h_out) {
-  if (len <= kPwLeaf) {
-    const int id = next_id++;
-    leaves.push_back(make_int4(id, begin, len, 0));
-    *h_out = 0;
-    return id;
-  }
-  int n2 = len / 2;
-  n2 -= n2 % 8;
-  int hl = 0, hr = 0;
-  const int l = pw_build(begin, n2, leaves, inner, height, next_id, &hl);
-  const int r = pw_build(begin + n2, len - n2, leaves, inner, height, next_id, &hr);
-  const int id = next_id++;
-  inner.push_back(make_int4(id, l, r, 0));
-  height.push_back(1 + std::max(hl, hr));
-  *h_out = height.back();
-  return id;
+// One step up the tree: a node without a right part is its left part.
+__device__ __forceinline__ void pw_up(float& v, bool h, unsigned lanes, int o) {
+  const float r = __shfl_down_sync(lanes, v, o);
+  const int has = __shfl_down_sync(lanes, (int)h, o);
+  if (has) v = __fadd_rn(v, r);
 }
 
-PwTree pw_tree(int n) {
-  PwTree t;
-  std::vector<int4> raw;
-  std::vector<int> h;
-  int next = 0, top = 0;
-  t.root = pw_build(0, n, t.leaves, raw, h, next, &top);
-  t.n_nodes = next;
-  std::vector<std::vector<int4>> by_level(top + 1);
-  for (size_t i = 0; i < raw.size(); ++i) by_level[h[i]].push_back(raw[i]);
-  for (int lv = 1; lv <= top; ++lv) {
-    t.inner.insert(t.inner.end(), by_level[lv].begin(), by_level[lv].end());
-    t.level_end.push_back((int)t.inner.size());
-  }
-  return t;
-}
-
-// Leaves of every segment w (data x + w * seg_stride): mode 0 sums x, mode 1
-// sums (x - centre[w])^2 with NumPy's float32 subtract and multiply.
-__global__ void pw_leaves_kernel(const float* __restrict__ x, long long seg_stride, int mode,
-                                 const float* __restrict__ centre, const int4* __restrict__ leaves,
-                                 int n_leaves, int n_nodes, int n_seg, float* __restrict__ vals) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= n_leaves) return;
-  const int4 lf = leaves[l];
-  for (int w = blockIdx.y; w < n_seg; w += gridDim.y) {
-    const float* base = x + (size_t)w * seg_stride + lf.y;
-    float s;
-    if (mode == 0) {
-      s = pw_leaf([&](int i) { return base[i]; }, lf.z);
-    } else {
-      const float c = centre[w];
-      s = pw_leaf(
-          [&](int i) {
-            const float d = __fsub_rn(base[i], c);
-            return __fmul_rn(d, d);
-          },
-          lf.z);
-    }
-    vals[(size_t)w * n_nodes + lf.x] = s;
-  }
-}
-
-// Inner nodes of every segment, one block per segment, level by level; then
-// out[w] = (0 + root) / count as NumPy's mean / var store it.
-__global__ void pw_inner_kernel(const int4* __restrict__ inner, const int* __restrict__ level_end,
-                                int n_levels, int n_nodes, int root, int count, int n_seg,
-                                float* __restrict__ vals, float* __restrict__ out) {
-  for (int w = blockIdx.x; w < n_seg; w += gridDim.x) {
-    float* v = vals + (size_t)w * n_nodes;
-    int begin = 0;
-    for (int lv = 0; lv < n_levels; ++lv) {
-      const int end = level_end[lv];
-      for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const int4 nd = inner[i];
-        v[nd.x] = __fadd_rn(v[nd.y], v[nd.z]);
+// The sum of `count` (a power of two) paths' nodes at their common root: a warp
+// for 32 of them at a time, in shared memory.
+__device__ float pw_join(float* val, unsigned char* has, int count) {
+  const int lane = threadIdx.x & 31;
+  while (count > 1) {
+    for (int i0 = 0; i0 < count; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      bool h = i < count && has[i];
+      float v = h ? val[i] : 0.0f;
+#pragma unroll
+      for (int o = 1; o < 32; o *= 2) pw_up(v, h, kFull, o);
+      __syncthreads();
+      if (lane == 0 && i < count) {
+        val[i / 32] = v;
+        has[i / 32] = h;
       }
-      begin = end;
       __syncthreads();
     }
-    if (threadIdx.x == 0) out[w] = np_divide_count(__fadd_rn(0.0f, v[root]), count);
+    count = (count + 31) / 32;
+  }
+  return val[0];
+}
+
+// Mean (mode 0) or population variance (mode 1, given the means; its root when
+// `root`) of segments of `len` values that start every seg_stride values, as
+// NumPy's mean / var store them.  Block (b, w) sums the 1 << lower paths below
+// path b of the upper `upper` turns of segment w's tree, and the last of a
+// segment's blocks joins their sums.  Eight lanes take a leaf, one of its eight
+// strided partial sums each; adding the partial sums by exchange is NumPy's
+// order, since a rounded addition commutes.
+// What bounds it is latency: on 2.16 million samples a launch takes 13 us where
+// a thread per leaf and a second launch for the inner nodes, level by level from
+// tables in global memory, took 46.
+constexpr int kPwThreads = 1024, kPwSlots = kPwThreads / 8;
+__global__ void __launch_bounds__(kPwThreads)
+pw_kernel(const float* __restrict__ x, long long seg_stride, int len, int n_seg, int mode,
+          const float* __restrict__ centre, int upper, int lower, bool root,
+          float* __restrict__ parts, int* __restrict__ tickets, float* __restrict__ out) {
+  // a sum per warp and kPwSlots paths, or one per block; then their flags
+  extern __shared__ float pw_val[];
+  __shared__ PwNode nodes[kPwSlots];
+  __shared__ bool last;
+  const int slots = 1 << lower, blocks = 1 << upper;
+  const int sums = max(slots / kPwSlots, 1) * (kPwThreads / 32);
+  unsigned char* has = reinterpret_cast<unsigned char*>(pw_val + max(sums, blocks));
+  const int tid = threadIdx.x, lane = tid & 7;
+  const unsigned group = 0xFFu << (tid & 24);  // of the warp's lanes
+  for (int w = blockIdx.y; w < n_seg; w += gridDim.y) {
+    const float* base = x + (size_t)w * seg_stride;
+    const float c = mode ? centre[w] : 0.0f;
+    auto get = [&](int i) {
+      const float v = base[i];
+      if (!mode) return v;
+      const float d = __fsub_rn(v, c);
+      return __fmul_rn(d, d);
+    };
+    for (int s0 = 0; s0 < slots; s0 += kPwSlots) {
+      if (tid < kPwSlots)
+        nodes[tid] = s0 + tid < slots
+                         ? PwNode{0, len}.down((int)(blockIdx.x << lower) + s0 + tid,
+                                               upper + lower)
+                         : PwNode{0, 0};
+      __syncthreads();
+      const PwNode nd = nodes[tid / 8];
+      float r = 0.0f;
+      if (nd.len >= 8) {
+        // the lane's values and the leaf's tail, loaded before they are added
+        const int rows = nd.len / 8, tail = nd.len % 8, lim = nd.begin + nd.len - tail;
+        float v[kPwLeaf / 8], t[7];
+#pragma unroll
+        for (int i = 0; i < kPwLeaf / 8; ++i)
+          v[i] = i < rows ? get(nd.begin + 8 * i + lane) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) t[i] = i < tail ? get(lim + i) : 0.0f;
+        r = v[0];
+#pragma unroll
+        for (int i = 1; i < kPwLeaf / 8; ++i)
+          if (i < rows) r = __fadd_rn(r, v[i]);
+        r = __fadd_rn(r, __shfl_xor_sync(group, r, 1));
+        r = __fadd_rn(r, __shfl_xor_sync(group, r, 2));
+        r = __fadd_rn(r, __shfl_xor_sync(group, r, 4));
+#pragma unroll
+        for (int i = 0; i < 7; ++i)
+          if (i < tail) r = __fadd_rn(r, t[i]);
+      } else {
+        for (int i = 0; i < nd.len; ++i) r = __fadd_rn(r, get(nd.begin + i));
+      }
+      __syncwarp();
+      const bool h = nd.len > 0;
+      pw_up(r, h, kFull, 8);  // the warp's four leaves
+      pw_up(r, h, kFull, 16);
+      if ((tid & 31) == 0) {
+        const int at = s0 / kPwSlots * (kPwThreads / 32) + tid / 32;
+        pw_val[at] = r;
+        has[at] = h;
+      }
+      __syncthreads();
+    }
+    float sum = pw_join(pw_val, has, sums);
+    bool write = tid == 0;
+    if (blocks > 1) {
+      if (tid == 0) {
+        parts[(size_t)w * blocks + blockIdx.x] = sum;
+        __threadfence();
+        last = atomicAdd(&tickets[w], 1) == blocks - 1;
+      }
+      __syncthreads();
+      if (last) {
+        __threadfence();
+        for (int b = tid; b < blocks; b += kPwThreads) {
+          pw_val[b] = __ldcg(parts + (size_t)w * blocks + b);
+          has[b] = PwNode{0, len}.down(b, upper).len > 0;
+        }
+        __syncthreads();
+        sum = pw_join(pw_val, has, blocks);
+      }
+      write = write && last;
+    }
+    if (write) {
+      const float v = np_divide_count(__fadd_rn(0.0f, sum), len);
+      out[w] = root ? __fsqrt_rn(v) : v;
+    }
     __syncthreads();
   }
 }
 
-// out[w] = mean (mode 0) or population variance (mode 1, given the means) of
-// segments of `len` values starting every seg_stride values.
-// Split trees of the lengths seen so far, built and uploaded once per device
-// and kept for the life of the process (up to kTreeCache lengths; beyond
-// that a tree is uploaded into the call's scratch).  The upload is ordered
-// on the call's stream and waited for (a plain cudaMemcpy from pageable
-// memory may return before its DMA lands), so a cached tree is complete
-// before any stream uses it.
-struct DevTree {
-  int n_leaves = 0, n_inner = 0, n_levels = 0, n_nodes = 0, root = 0;
-  const int4* leaves = nullptr;
-  const int4* inner = nullptr;
-  const int* levels = nullptr;
-};
-constexpr size_t kTreeCache = 64;
-std::mutex g_tree_mu;
-std::map<std::pair<int, int>, DevTree> g_trees;
-
-int upload_tree(const PwTree& t, DevTree* d, void* mem, cudaStream_t st) {
-  char* p = static_cast<char*>(mem);
-  d->n_leaves = (int)t.leaves.size();
-  d->n_inner = (int)t.inner.size();
-  d->n_levels = (int)t.level_end.size();
-  d->n_nodes = t.n_nodes;
-  d->root = t.root;
-  d->leaves = reinterpret_cast<const int4*>(p);
-  d->inner = reinterpret_cast<const int4*>(p + t.leaves.size() * sizeof(int4));
-  d->levels = reinterpret_cast<const int*>(p + (t.leaves.size() + t.inner.size()) *
-                                                   sizeof(int4));
-  BP_CUDA(cudaMemcpyAsync(p, t.leaves.data(), t.leaves.size() * sizeof(int4),
-                          cudaMemcpyHostToDevice, st));
-  if (!t.inner.empty()) {
-    BP_CUDA(cudaMemcpyAsync(p + t.leaves.size() * sizeof(int4), t.inner.data(),
-                            t.inner.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-    BP_CUDA(cudaMemcpyAsync(p + (t.leaves.size() + t.inner.size()) * sizeof(int4),
-                            t.level_end.data(), t.level_end.size() * sizeof(int),
-                            cudaMemcpyHostToDevice, st));
-  }
-  // the host vectors are freed on return and a cached tree is shared by
-  // every stream: wait until the copies have landed
-  BP_CUDA(cudaStreamSynchronize(st));
-  return BP_OK;
-}
-
-size_t tree_bytes(const PwTree& t) {
-  return (t.leaves.size() + t.inner.size()) * sizeof(int4) + t.level_end.size() * sizeof(int) +
-         16;
-}
-
-int get_tree(int len, DevTree* out, Scratch& sc) {
-  int dev = 0;
-  BP_CUDA(cudaGetDevice(&dev));
-  const auto key = std::make_pair(dev, len);
-  {
-    std::lock_guard<std::mutex> lock(g_tree_mu);
-    auto it = g_trees.find(key);
-    if (it != g_trees.end()) {
-      *out = it->second;
-      return BP_OK;
-    }
-  }
-  const PwTree t = pw_tree(len);
-  std::lock_guard<std::mutex> lock(g_tree_mu);
-  auto it = g_trees.find(key);
-  if (it != g_trees.end()) {
-    *out = it->second;
-    return BP_OK;
-  }
-  void* mem = nullptr;
-  if (g_trees.size() < kTreeCache) {
-    BP_CUDA(cudaMalloc(&mem, tree_bytes(t)));
-    DevTree d;
-    if (int rc = upload_tree(t, &d, mem, sc.st)) {
-      cudaFree(mem);
-      return rc;
-    }
-    g_trees.emplace(key, d);
-    *out = d;
-    return BP_OK;
-  }
-  char* scratch = nullptr;  // cache full: this call's own copy
-  BP_TRY(sc.get(&scratch, tree_bytes(t)));
-  return upload_tree(t, out, scratch, sc.st);  // ordered after the allocation
-}
-
+// tickets: n_seg zeros, for this call alone.
 int pw_mean(const float* x, long long seg_stride, int len, int n_seg, int mode,
-            const float* centre, float* out, Scratch& sc, cudaStream_t st) {
-  DevTree t;
-  BP_TRY(get_tree(len, &t, sc));
-  float* vals = nullptr;
-  BP_TRY(sc.get(&vals, (size_t)t.n_nodes * n_seg));
-  dim3 g1((t.n_leaves + 127) / 128, (unsigned)std::min(n_seg, 65535));
-  pw_leaves_kernel<<<g1, 128, 0, st>>>(x, seg_stride, mode, centre, t.leaves, t.n_leaves,
-                                       t.n_nodes, n_seg, vals);
-  BP_LAUNCHED("pw_leaves_kernel");
-  pw_inner_kernel<<<(unsigned)std::min(n_seg, 65535), n_seg == 1 ? 1024 : 256, 0, st>>>(
-      t.inner, t.levels, t.n_levels, t.n_nodes, t.root, len, n_seg, vals, out);
-  BP_LAUNCHED("pw_inner_kernel");
+            const float* centre, bool root, float* out, Scratch& sc, cudaStream_t st) {
+  const int depth = pw_depth(len);
+  // 128 leaves per block, at most 256 blocks per segment, at most 4,096 leaves
+  // per block: 2.16 million samples have 32,768
+  const int lower = std::min(std::max(std::min(depth, 7), depth - 8), 12), upper = depth - lower;
+  const size_t sums = std::max(std::max((1 << lower) / kPwSlots, 1) * (kPwThreads / 32), 1 << upper);
+  const size_t smem = sums * (sizeof(float) + 1);
+  float* parts = nullptr;
+  int* tickets = nullptr;
+  if (upper > 0) {
+    BP_TRY(sc.get(&parts, (size_t)n_seg << upper));
+    BP_TRY(sc.get(&tickets, n_seg));
+    BP_CUDA(cudaMemsetAsync(tickets, 0, (size_t)n_seg * sizeof(int), st));
+  }
+  pw_kernel<<<dim3(1u << upper, (unsigned)std::min(n_seg, 65535)), kPwThreads, smem, st>>>(
+      x, seg_stride, len, n_seg, mode, centre, upper, lower, root, parts, tickets, out);
+  BP_LAUNCHED("pw_kernel");
   return BP_OK;
+}
+
+// ---- bit masks over the samples ------------------------------------------------
+// One bit per sample and the number set per kMaskBlock samples.  A compaction
+// then is a launch that sets the bits, one that scans the counts (a single
+// block) and one that takes the set bits with their ranks.  (With flags and ranks
+// as integers per sample, the compaction of 2.16 million samples moved 35 MB and
+// took 35 us.)
+constexpr int kMaskRows = 16, kMaskThreads = 256;
+constexpr int kMaskBlock = kMaskThreads * kMaskRows;  // 32 samples per word, 16 words per warp
+
+struct Mask {
+  unsigned* bits;
+  int* counts;  // per block; after scan_counts the set bits before it, and all of them
+  int n_words, n_blocks;
+};
+int get_mask(Mask* m, int n, Scratch& sc) {
+  m->n_words = (int)(((long long)n + 31) / 32);
+  m->n_blocks = (int)(((long long)n + kMaskBlock - 1) / kMaskBlock);
+  BP_TRY(sc.get(&m->bits, m->n_words));
+  return sc.get(&m->counts, (size_t)m->n_blocks + 1);
+}
+
+// The block's bits and count: flag(i, v, r) for its samples, v their values in
+// the thread's rows (loaded before any is looked at), v[r] the sample's.
+template <class Flag>
+__device__ void mask_set(const float* __restrict__ x, int n, const Mask& m, const Flag& flag) {
+  __shared__ int total;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned base = (blockIdx.x * (kMaskThreads / 32) + warp) * 32u * kMaskRows;
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  float v[kMaskRows];
+#pragma unroll
+  for (int r = 0; r < kMaskRows; ++r) {
+    const unsigned i = base + r * 32 + lane;
+    v[r] = i < (unsigned)n ? x[i] : 0.0f;
+  }
+  unsigned word = 0;
+#pragma unroll
+  for (int r = 0; r < kMaskRows; ++r) {
+    const unsigned i = base + r * 32 + lane;
+    const bool f = flag(i, v, r);
+    const unsigned b = __ballot_sync(kFull, i < (unsigned)n && f);
+    if (lane == r) word = b;
+  }
+  const unsigned at = base / 32 + lane;
+  if (lane < kMaskRows && at < (unsigned)m.n_words) m.bits[at] = word;
+  const int c = __reduce_add_sync(kFull, __popc(word));
+  if (lane == 0 && c) atomicAdd(&total, c);
+  __syncthreads();
+  if (threadIdx.x == 0) m.counts[blockIdx.x] = total;
+}
+
+// counts -> the counts before each block, and the total behind the last.
+__global__ void __launch_bounds__(1024) scan_counts_kernel(int* __restrict__ counts, int n) {
+  __shared__ int warp_sum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int each = (n + 1023) / 1024;
+  const int b = min(tid * each, n), e = min(b + each, n);
+  int mine = 0;
+  for (int i = b; i < e; ++i) mine += counts[i];
+  int sum = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(kFull, sum, o);
+    if (lane >= o) sum += v;
+  }
+  if (lane == 31) warp_sum[warp] = sum;
+  __syncthreads();
+  const int from = __reduce_add_sync(kFull, lane < warp ? warp_sum[lane] : 0);
+  int run = from + sum - mine;
+  for (int i = b; i < e; ++i) {
+    const int c = counts[i];
+    counts[i] = run;
+    run += c;
+  }
+  if (tid == 1023) counts[n] = run;
+}
+int scan_counts(const Mask& m, cudaStream_t st) {
+  scan_counts_kernel<<<1, 1024, 0, st>>>(m.counts, m.n_blocks);
+  BP_LAUNCHED("scan_counts_kernel");
+  return BP_OK;
+}
+
+// take(i, v, set, rank) for the block's samples: rank = set bits before i, v =
+// load(i, set, rank), loaded for all of the thread's rows before any is taken.
+template <class Load, class Take>
+__device__ void mask_take(int n, const Mask& m, const Load& load, const Take& take) {
+  __shared__ int warp_sum[kMaskThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned low = (1u << lane) - 1u;
+  const unsigned base = (blockIdx.x * (kMaskThreads / 32) + warp) * 32u * kMaskRows;
+  const unsigned at = base / 32 + lane;
+  const unsigned word = lane < kMaskRows && at < (unsigned)m.n_words ? m.bits[at] : 0u;
+  int sum = __popc(word);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(kFull, sum, o);
+    if (lane >= o) sum += u;
+  }
+  if (lane == 31) warp_sum[warp] = sum;
+  __syncthreads();
+  int from = m.counts[blockIdx.x] + sum - __popc(word);  // before the lane's word
+#pragma unroll
+  for (int u = 0; u < kMaskThreads / 32; ++u) from += u < warp ? warp_sum[u] : 0;
+  float v[kMaskRows];
+#pragma unroll
+  for (int r = 0; r < kMaskRows; ++r) {
+    const unsigned w = __shfl_sync(kFull, word, r);
+    const int f = __shfl_sync(kFull, from, r);
+    const unsigned i = base + r * 32 + lane;
+    v[r] = i < (unsigned)n ? load((int)i, ((w >> lane) & 1u) != 0u, f + __popc(w & low)) : 0.0f;
+  }
+#pragma unroll
+  for (int r = 0; r < kMaskRows; ++r) {
+    const unsigned w = __shfl_sync(kFull, word, r);
+    const int f = __shfl_sync(kFull, from, r);
+    const unsigned i = base + r * 32 + lane;
+    if (i < (unsigned)n) take((int)i, v[r], ((w >> lane) & 1u) != 0u, f + __popc(w & low));
+  }
 }
 
 // ---- threshold kernels ---------------------------------------------------------
-__global__ void zero_flags_kernel(const float* __restrict__ x, int n, int* __restrict__ flags) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > n) return;
-  flags[i] = (i < n && x[i] == 0.0f) ? 1 : 0;
+__global__ void __launch_bounds__(kMaskThreads)
+zero_mask_kernel(const float* __restrict__ x, int n, Mask m) {
+  mask_set(x, n, m, [](unsigned, const float (&v)[kMaskRows], int r) { return v[r] == 0.0f; });
 }
 
 // Non-zero samples, in order, into nz.
-__global__ void gather_nonzero_kernel(const float* __restrict__ x, int n,
-                                      const int* __restrict__ zero_rank, float* __restrict__ nz) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float v = x[i];
-  if (v != 0.0f) nz[i - zero_rank[i]] = v;
+__global__ void __launch_bounds__(kMaskThreads)
+gather_nonzero_kernel(const float* __restrict__ x, int n, Mask zeros, float* __restrict__ nz) {
+  mask_take(
+      n, zeros, [&](int i, bool, int) { return x[i]; },
+      [&](int i, float v, bool zero, int rank) {
+        if (!zero) nz[i - rank] = v;
+      });
 }
 
 // SplitMix64 output function (Steele, Lea & Flood, OOPSLA 2014).
@@ -299,26 +392,21 @@ __global__ void normal_kernel(unsigned long long seed, int n, float* __restrict_
 }
 
 // Zeros replaced by noise * deviation + centre (NumPy float32 multiply, add).
-__global__ void fill_zeros_kernel(const float* __restrict__ x, int n,
-                                  const int* __restrict__ zero_rank,
-                                  const float* __restrict__ noise,
-                                  const float* __restrict__ centre0,
-                                  const float* __restrict__ dev0, float* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float v = x[i];
-  out[i] = v != 0.0f ? v : __fadd_rn(__fmul_rn(noise[zero_rank[i]], *dev0), *centre0);
+__global__ void __launch_bounds__(kMaskThreads)
+fill_zeros_kernel(const float* __restrict__ x, int n, Mask zeros,
+                  const float* __restrict__ noise, const float* __restrict__ centre0,
+                  const float* __restrict__ dev0, float* __restrict__ out) {
+  const float c = *centre0, d = *dev0;
+  mask_take(
+      n, zeros, [&](int i, bool zero, int rank) { return zero ? noise[rank] : x[i]; },
+      [&](int i, float v, bool zero, int) {
+        out[i] = zero ? __fadd_rn(__fmul_rn(v, d), c) : v;
+      });
 }
 
-// Default centre / deviation for the rms rule: deviation = sqrt(variance);
-// both NaN when there is no non-zero sample (NumPy's mean of nothing).
-__global__ void finish_stats_kernel(float* __restrict__ stats, int have) {
-  if (threadIdx.x != 0) return;
-  if (have) {
-    stats[1] = __fsqrt_rn(stats[1]);
-  } else {
-    stats[0] = stats[1] = __uint_as_float(0x7FC00000u);
-  }
+// NumPy's mean and deviation of nothing.
+__global__ void no_stats_kernel(float* __restrict__ stats) {
+  if (threadIdx.x < 2) stats[threadIdx.x] = __uint_as_float(0x7FC00000u);
 }
 
 // np.maximum on float32: NaN propagates, equal values give the second operand.
@@ -326,183 +414,243 @@ __device__ __forceinline__ float np_maximum(float a, float b) {
   return (a > b || isnan(a)) ? a : b;
 }
 
-// thr[w] = centre + num_dev * deviation (rms: deviation = sqrt(variance)).
-__global__ void window_threshold_kernel(const float* __restrict__ centre,
-                                        const float* __restrict__ spread, int n_win, int is_var,
-                                        float num_dev, float* __restrict__ thr) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n_win) return;
-  const float dev = is_var ? __fsqrt_rn(spread[w]) : spread[w];
-  thr[w] = __fadd_rn(centre[w], __fmul_rn(num_dev, dev));
-}
-
-// neighbour = -1: out[i] = max(in[i-1], in[i]) for i >= 1 (in[0] kept);
-// neighbour = +1: out[i] = max(in[i], in[i+1]) for i < n-1 (in[n-1] kept).
-__global__ void neighbour_max_kernel(const float* __restrict__ in, int n_win, int neighbour,
-                                     float* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_win) return;
-  float v = in[i];
-  if (neighbour < 0 && i >= 1) v = np_maximum(in[i - 1], in[i]);
-  if (neighbour > 0 && i + 1 < n_win) v = np_maximum(in[i], in[i + 1]);
-  out[i] = v;
-}
+// A window's threshold, centre + num_dev * deviation (rms: deviation =
+// sqrt(variance)), and the maximum over its neighbours as the tutorial takes it:
+// first with the window before, then of those with the window after.
+struct WindowThreshold {
+  const float *centre, *spread;
+  int n_win, is_var;
+  float num_dev;
+  __device__ float at(int w) const {
+    const float dev = is_var ? __fsqrt_rn(spread[w]) : spread[w];
+    return __fadd_rn(centre[w], __fmul_rn(num_dev, dev));
+  }
+  __device__ float with_before(int w) const {
+    return w >= 1 ? np_maximum(at(w - 1), at(w)) : at(w);
+  }
+  __device__ float with_both(int w) const {
+    return w + 1 < n_win ? np_maximum(with_before(w), with_before(w + 1)) : with_before(w);
+  }
+};
 
 // Per-sample threshold: windows' values at (half + j) / shift for the middle
 // samples, the first / last middle value repeated at both ends.
-__global__ void spread_threshold_kernel(const float* __restrict__ thr, int n_win, int n,
-                                        int window, int half, int shift, float* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const long long n_mid = (long long)n - window;
-  long long j = i - half;
-  if (j < 0) j = 0;
-  if (j > n_mid - 1) j = n_mid - 1;
-  long long idx = (half + j) / shift;
-  if (idx > n_win - 1) idx = n_win - 1;
-  out[i] = thr[idx];
+__global__ void __launch_bounds__(256)
+spread_threshold_kernel(WindowThreshold thr, int n, int window, int half, int shift,
+                        float* __restrict__ out) {
+  constexpr int U = 4;
+  const unsigned i0 = blockIdx.x * 256u * U + threadIdx.x;
+  const int n_mid = n - window;
+  unsigned done = ~0u;
+  float v = 0.0f;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const unsigned i = i0 + u * 256;
+    if (i >= (unsigned)n) return;
+    const int j = min(max((int)i - half, 0), n_mid - 1);
+    const unsigned w = min((unsigned)(half + j) / (unsigned)shift, (unsigned)thr.n_win - 1u);
+    if (w != done) v = thr.with_both((int)w);
+    done = w;
+    out[i] = v;
+  }
 }
 
 // ---- peak kernels ----------------------------------------------------------
 // Rising edges x[i-1] < x[i]: a peak at i when x[i+1] < x[i]; a plateau to
 // measure when x[i+1] == x[i].
-__global__ void local_max_kernel(const float* __restrict__ x, int n, int* __restrict__ flags,
-                                 int* __restrict__ plateau, int* __restrict__ n_plateau) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 1 || i >= (long long)n - 1) return;
-  const float xi = x[i];
-  if (!(x[i - 1] < xi)) return;
-  const float nx = x[i + 1];
-  if (nx < xi) {
-    flags[i] = 1;
-  } else if (nx == xi) {
-    plateau[atomicAdd(n_plateau, 1)] = (int)i;
-  }
+__global__ void __launch_bounds__(kMaskThreads)
+local_max_kernel(const float* __restrict__ x, int n, Mask peaks, int* __restrict__ plateau,
+                 int* __restrict__ n_plateau) {
+  const int lane = threadIdx.x & 31;
+  const unsigned base =
+      (blockIdx.x * (kMaskThreads / 32) + (threadIdx.x >> 5)) * 32u * kMaskRows;
+  // the samples before and after the warp's
+  const float first = base >= 1 && base - 1 < (unsigned)n ? x[base - 1] : 0.0f;
+  const unsigned end = base + 32 * kMaskRows;
+  const float last = end < (unsigned)n ? x[end] : 0.0f;
+  mask_set(x, n, peaks, [&](unsigned i, const float (&v)[kMaskRows], int r) {
+    float before = __shfl_up_sync(kFull, v[r], 1), after = __shfl_down_sync(kFull, v[r], 1);
+    const float row_before = r ? __shfl_sync(kFull, v[r ? r - 1 : 0], 31) : first;
+    const float row_after =
+        r + 1 < kMaskRows ? __shfl_sync(kFull, v[r + 1 < kMaskRows ? r + 1 : r], 0) : last;
+    if (lane == 0) before = row_before;
+    if (lane == 31) after = row_after;
+    if (i < 1 || i >= (unsigned)n - 1 || !(before < v[r])) return false;
+    if (after == v[r]) plateau[atomicAdd(n_plateau, 1)] = (int)i;
+    return after < v[r];
+  });
 }
 
-// One warp per plateau starting at i: its end j is the first index > i with
+// A warp per plateau starting at i: its end j is the first index > i with
 // x[j] != x[i], capped at n - 1; a peak at (i + j - 1) / 2 when x[j] < x[i].
-__global__ void plateau_kernel(const float* __restrict__ x, int n, const int* __restrict__ plateau,
-                               const int* __restrict__ n_plateau, int* __restrict__ flags) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= *n_plateau) return;
-  const int i = plateau[gw];
-  const float xi = x[i];
-  for (long long base = (long long)i + 1;; base += 32) {
-    const long long j = base + lane;
-    const bool stop = j >= (long long)n - 1 || x[j] != xi;
-    const unsigned b = __ballot_sync(kFull, stop);
-    if (b) {
-      long long e = base + __ffs(b) - 1;
-      if (e > n - 1) e = n - 1;
-      if (lane == 0 && x[e] < xi) flags[(i + e - 1) / 2] = 1;
-      return;
-    }
-  }
-}
-
-__global__ void scatter_flagged_kernel(const int* __restrict__ flags, const int* __restrict__ rank,
-                                       int n, int* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (flags[i]) out[rank[i]] = (int)i;
-}
-
-__global__ void gather_heights_kernel(const float* __restrict__ x, const int* __restrict__ pos,
-                                      int m, float* __restrict__ val, int* __restrict__ state,
-                                      int* __restrict__ undecided) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  val[j] = x[pos[j]];
-  state[j] = 0;
-  undecided[j] = j;
-}
-
-enum : int { kUndecided = 0, kKept = 1, kDropped = 2 };
-
-// Peak k goes before peak j in SciPy's order (decreasing height; the later
-// sample first among equal heights, as a stable ascending sort read backwards).
-__device__ __forceinline__ bool before(const float* val, int k, int j) {
-  return val[k] > val[j] || (val[k] == val[j] && k > j);
-}
-
-// Round step 1, one warp per undecided peak: kept when no undecided peak
-// within the distance goes before it.
-__global__ void distance_keep_kernel(const int* __restrict__ pos, const float* __restrict__ val,
-                                     const int* __restrict__ state, int m, long long dist,
-                                     const int* __restrict__ undecided, int n_undecided,
-                                     int* __restrict__ kept, int* __restrict__ n_kept) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= n_undecided) return;
-  const int j = undecided[gw];
-  const long long pj = pos[j];
-  bool blocked = false;
-  for (long long base = (long long)j - 1; base >= 0; base -= 32) {
-    const long long k = base - lane;
-    const bool in = k >= 0 && pj - pos[k] < dist;
-    const bool blk = in && state[k] == kUndecided && before(val, (int)k, j);
-    if (__any_sync(kFull, blk)) {
-      blocked = true;
-      break;
-    }
-    if (__any_sync(kFull, !in)) break;
-  }
-  if (!blocked) {
-    for (long long base = (long long)j + 1; base < m; base += 32) {
-      const long long k = base + lane;
-      const bool in = k < m && pos[k] - pj < dist;
-      const bool blk = in && state[k] == kUndecided && before(val, (int)k, j);
-      if (__any_sync(kFull, blk)) {
-        blocked = true;
+__global__ void __launch_bounds__(256)
+plateau_kernel(const float* __restrict__ x, int n, const int* __restrict__ plateau,
+               const int* __restrict__ n_plateau, Mask peaks) {
+  const int lane = threadIdx.x & 31, total = *n_plateau;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total; w += warps) {
+    const int i = plateau[w];
+    const float xi = x[i];
+    for (long long base = (long long)i + 1;; base += 32) {
+      const long long j = base + lane;
+      const bool stop = j >= (long long)n - 1 || x[j] != xi;
+      const unsigned b = __ballot_sync(kFull, stop);
+      if (b) {
+        long long e = base + __ffs(b) - 1;
+        if (e > n - 1) e = n - 1;
+        if (lane == 0 && x[e] < xi) {
+          const int p = (int)((i + e - 1) / 2);
+          atomicOr(&peaks.bits[p >> 5], 1u << (p & 31));
+          atomicAdd(&peaks.counts[p / kMaskBlock], 1);
+        }
         break;
       }
-      if (__any_sync(kFull, !in)) break;
     }
   }
-  if (!blocked && lane == 0) kept[atomicAdd(n_kept, 1)] = j;
 }
 
-// Round step 2, one warp per newly kept peak: mark it kept and drop every
-// undecided peak within the distance.
-__global__ void distance_drop_kernel(const int* __restrict__ pos, int* __restrict__ state, int m,
-                                     long long dist, const int* __restrict__ kept,
-                                     const int* __restrict__ n_kept) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void __launch_bounds__(kMaskThreads)
+positions_kernel(int n, Mask m, int* __restrict__ out) {
+  mask_take(n, m, [](int, bool, int) { return 0.0f; }, [&](int i, float, bool set, int rank) {
+    if (set) out[rank] = i;
+  });
+}
+
+// SciPy's distance rule, one cooperative launch for all of its rounds.
+struct Peak {
+  int pos;
+  float val;  // -infinity once it is dropped (a peak is above its neighbours)
+};
+struct Distance {
+  const float* x;
+  const int* pos;      // peaks, ascending
+  const int* n_peaks;  // on the device
+  int dist;
+  const float* above;  // peaks that are not above it are left out of `out`; may be NULL
+  Peak* peaks;
+  int *list, *list2, *kept;  // per peak
+  int* counters;             // 6
+  Mask out;                  // the kept peaks
+};
+
+// A round: every undecided peak with no undecided one before it within the
+// distance is kept, and then what is undecided within the distance of a kept one
+// is dropped.  (Before it, in SciPy's order: higher, or as high and later -- a
+// stable ascending sort read backwards.  No kept peak lies within the distance
+// of an undecided one.)  A lane looks at the nearest kNear peaks on both sides of
+// its own, which block sixteen peaks in seventeen; a warp then looks along for
+// each that is left.
+// What bounds it is the latency of the rounds: two grid barriers and a few
+// dependent reads each.  On 2.16 million samples with 538,000 peaks it takes
+// 86 us; a warp per peak, three launches and a read-back per round took 420.
+constexpr int kNear = 8, kDistThreads = 1024;
+__global__ void __launch_bounds__(kDistThreads) distance_kernel(Distance a) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   const int lane = threadIdx.x & 31;
-  if (gw >= *n_kept) return;
-  const int j = kept[gw];
-  const long long pj = pos[j];
-  if (lane == 0) state[j] = kKept;
-  for (long long base = (long long)j - 1; base >= 0; base -= 32) {
-    const long long k = base - lane;
-    const bool in = k >= 0 && pj - pos[k] < dist;
-    if (in && state[k] == kUndecided) state[k] = kDropped;
-    if (__any_sync(kFull, !in)) break;
+  const int thread = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  const int warp = thread >> 5, warps = threads >> 5;
+  const unsigned before_lane = (1u << lane) - 1u;
+  const int m = *a.n_peaks;
+  for (int j = thread; j < m; j += threads) a.peaks[j] = Peak{a.pos[j], a.x[a.pos[j]]};
+  for (int w = thread; w < a.out.n_words; w += threads) a.out.bits[w] = 0u;
+  for (int b = thread; b < a.out.n_blocks; b += threads) a.out.counts[b] = 0;
+  if (thread < 6) a.counters[thread] = 0;
+  grid.sync();
+  // The peak, or where there is none one that is too far and blocks nothing.
+  auto peak = [&](int k) {
+    if (k < 0 || k >= m) return make_int2(k < 0 ? INT_MIN : INT_MAX, 0xFF800000);
+    return *reinterpret_cast<const int2*>(a.peaks + k);
+  };
+  // A peak's window is lo < position < hi; no end lies beyond those of peak().
+  auto window_lo = [&](int p) { return (int)max((long long)p - a.dist, (long long)INT_MIN); };
+  auto window_hi = [&](int p) { return (int)min((long long)p + a.dist, (long long)INT_MAX); };
+  int u = m;
+  int *list = nullptr, *next = a.list, *spare = a.list2;
+  for (int round = 0; u > 0 && round <= m; ++round) {
+    int* n_kept = a.counters + round % 3;
+    int* n_next = a.counters + 3 + round % 3;
+    for (int t = warp; t < (u + 31) / 32; t += warps) {
+      const int i = t * 32 + lane;
+      const int j = i >= u ? -1 : list ? list[i] : i;
+      const int2 mine = peak(j);
+      const float vj = __int_as_float(mine.y);
+      const bool open = vj > __int_as_float(0xFF800000);
+      const int lo = window_lo(mine.x), hi = window_hi(mine.x);
+      bool blocked = false, left = false, right = false;
+      if (open) {
+        int2 l[kNear], r[kNear];
+#pragma unroll
+        for (int d = 0; d < kNear; ++d) {
+          l[d] = peak(j - 1 - d);
+          r[d] = j < m - 1 - d ? peak(j + 1 + d) : make_int2(INT_MAX, 0xFF800000);
+        }
+#pragma unroll
+        for (int d = 0; d < kNear; ++d) {
+          blocked |= l[d].x > lo && __int_as_float(l[d].y) > vj;
+          blocked |= r[d].x < hi && __int_as_float(r[d].y) >= vj;
+        }
+        left = !blocked && l[kNear - 1].x > lo;
+        right = !blocked && r[kNear - 1].x < hi;
+      }
+      unsigned rest = __ballot_sync(kFull, left || right);
+      while (rest) {
+        const int src = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const int jj = __shfl_sync(kFull, j, src);
+        const float vv = __shfl_sync(kFull, vj, src);
+        const int ll = __shfl_sync(kFull, lo, src), hh = __shfl_sync(kFull, hi, src);
+        bool go_l = __shfl_sync(kFull, (int)left, src) != 0;
+        bool go_r = __shfl_sync(kFull, (int)right, src) != 0;
+        bool hit = false;
+        for (int d = kNear + 1 + lane; (go_l || go_r) && !hit; d += 32) {
+          const int2 l = go_l && d <= jj ? peak(jj - d) : make_int2(INT_MIN, 0xFF800000);
+          const int2 r = go_r && d < m - jj ? peak(jj + d) : make_int2(INT_MAX, 0xFF800000);
+          hit = __any_sync(kFull, (l.x > ll && __int_as_float(l.y) > vv) ||
+                                      (r.x < hh && __int_as_float(r.y) >= vv));
+          go_l = __all_sync(kFull, l.x > ll);
+          go_r = __all_sync(kFull, r.x < hh);
+        }
+        if (lane == src) blocked = hit;
+      }
+      const unsigned keep = __ballot_sync(kFull, open && !blocked);
+      const unsigned stay = __ballot_sync(kFull, open && blocked);
+      int k0 = 0, s0 = 0;
+      if (lane == 0) {
+        if (keep) k0 = atomicAdd(n_kept, __popc(keep));
+        if (stay) s0 = atomicAdd(n_next, __popc(stay));
+      }
+      k0 = __shfl_sync(kFull, k0, 0);
+      s0 = __shfl_sync(kFull, s0, 0);
+      if (open && !blocked) a.kept[k0 + __popc(keep & before_lane)] = j;
+      if (open && blocked) next[s0 + __popc(stay & before_lane)] = j;
+    }
+    grid.sync();
+    const int nk = *(volatile int*)n_kept;
+    for (int t = warp; t < nk; t += warps) {
+      const int j = a.kept[t], pj = a.peaks[j].pos;
+      const int lo = window_lo(pj), hi = window_hi(pj);
+      if (lane == 0 && (!a.above || a.x[pj] > a.above[pj])) {
+        atomicOr(&a.out.bits[pj >> 5], 1u << (pj & 31));
+        atomicAdd(&a.out.counts[pj / kMaskBlock], 1);
+      }
+      bool go_l = true, go_r = true;
+      for (int d = 1 + lane; go_l || go_r; d += 32) {
+        const bool l = go_l && d <= j && a.peaks[j - d].pos > lo;
+        const bool r = go_r && d < m - j && a.peaks[j + d].pos < hi;
+        if (l) a.peaks[j - d].val = __int_as_float(0xFF800000);
+        if (r) a.peaks[j + d].val = __int_as_float(0xFF800000);
+        go_l = __all_sync(kFull, l);
+        go_r = __all_sync(kFull, r);
+      }
+    }
+    // the counters of the next round: last read a round ago
+    if (thread < 2) a.counters[3 * thread + (round + 1) % 3] = 0;
+    grid.sync();
+    u = *(volatile int*)n_next;
+    list = next;
+    next = spare;
+    spare = list;
   }
-  for (long long base = (long long)j + 1; base < m; base += 32) {
-    const long long k = base + lane;
-    const bool in = k < m && pos[k] - pj < dist;
-    if (in && state[k] == kUndecided) state[k] = kDropped;
-    if (__any_sync(kFull, !in)) break;
-  }
-}
-
-// Round step 3: the still undecided peaks form the next work list.
-__global__ void distance_next_kernel(const int* __restrict__ state,
-                                     const int* __restrict__ undecided, int n_undecided,
-                                     int* __restrict__ next, int* __restrict__ n_next) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_undecided) return;
-  const int j = undecided[i];
-  if (state[j] == kUndecided) next[atomicAdd(n_next, 1)] = j;
-}
-
-__global__ void kept_flags_kernel(const int* __restrict__ state, int m, int* __restrict__ flags) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j > m) return;
-  flags[j] = (j < m && state[j] == kKept) ? 1 : 0;
 }
 
 __global__ void above_flags_kernel(const float* __restrict__ x, const float* __restrict__ thr,
@@ -526,6 +674,18 @@ __global__ void scatter_detections_kernel(const int* __restrict__ flags,
   out_peaks[r] = p;
   if (out_heights) out_heights[r] = x[p];
   if (argmax && out_sources) out_sources[r] = argmax[p];
+}
+
+__global__ void __launch_bounds__(kMaskThreads)
+mask_detections_kernel(int n, Mask m, const float* __restrict__ x,
+                       const int32_t* __restrict__ argmax, int32_t* __restrict__ out_peaks,
+                       float* __restrict__ out_heights, int32_t* __restrict__ out_sources) {
+  mask_take(n, m, [](int, bool, int) { return 0.0f; }, [&](int i, float, bool set, int r) {
+    if (!set) return;
+    out_peaks[r] = i;
+    if (out_heights) out_heights[r] = x[i];
+    if (argmax && out_sources) out_sources[r] = argmax[i];
+  });
 }
 
 // ---- host drivers -------------------------------------------------------------
@@ -667,12 +827,15 @@ struct PeakOut {
 };
 
 // Keeps the entries of `pos` (m, device) whose flag is set, in order, into a
-// new scratch array; returns their number.
-int keep_flagged(int* flags, int m, int** pos, Scratch& sc, cudaStream_t st, int* kept) {
+// new scratch array; returns their number
+// and where it is on the device.
+int keep_flagged(int* flags, int m, int** pos, Scratch& sc, cudaStream_t st, int* kept,
+                 const int** d_kept) {
   int* rank = nullptr;
   int* out = nullptr;
   BP_TRY(sc.get(&rank, (size_t)m + 1));
   BP_TRY(scan_flags(flags, rank, m, sc, st));
+  *d_kept = rank + m;
   BP_TRY(read_back(kept, rank + m, st));
   BP_TRY(sc.get(&out, std::max(*kept, 1)));
   compact_peaks_kernel<<<grid_for(m, 256), 256, 0, st>>>(flags, rank, m, *pos, nullptr, nullptr,
@@ -683,41 +846,80 @@ int keep_flagged(int* flags, int m, int** pos, Scratch& sc, cudaStream_t st, int
   return BP_OK;
 }
 
+// Local maxima of x (plateaus by their midpoint) as a mask with scanned counts.
+int local_maxima(const float* x, int n, Mask* peaks, Scratch& sc, cudaStream_t st) {
+  int *plateau = nullptr, *n_plateau = nullptr;
+  BP_TRY(get_mask(peaks, n, sc));
+  BP_TRY(sc.get(&plateau, (size_t)n / 2 + 1));  // a rising edge and an equal sample each
+  BP_TRY(sc.get(&n_plateau, 1));
+  BP_CUDA(cudaMemsetAsync(n_plateau, 0, sizeof(int), st));
+  local_max_kernel<<<(unsigned)peaks->n_blocks, kMaskThreads, 0, st>>>(x, n, *peaks, plateau,
+                                                                      n_plateau);
+  BP_LAUNCHED("local_max_kernel");
+  plateau_kernel<<<(unsigned)std::min(peaks->n_blocks, 148), 256, 0, st>>>(x, n, plateau,
+                                                                           n_plateau, *peaks);
+  BP_LAUNCHED("plateau_kernel");
+  return scan_counts(*peaks, st);
+}
+
+// The distance rule on the peaks pos[0 .. *d_m - 1] (at most `cap`, on the
+// device): the kept ones as a mask with scanned counts.
+int distance_rule(const float* x, int n, const int* pos, const int* d_m, int cap, double distance,
+                  const float* above, Mask* out, Scratch& sc, cudaStream_t st) {
+  const double dc = std::ceil(distance);
+  Distance a{};
+  a.x = x;
+  a.pos = pos;
+  a.n_peaks = d_m;
+  a.dist = dc > (double)n ? n + 1 : (int)dc;
+  a.above = above;
+  BP_TRY(sc.get(&a.peaks, cap));
+  BP_TRY(sc.get(&a.list, cap));
+  BP_TRY(sc.get(&a.list2, cap));
+  BP_TRY(sc.get(&a.kept, cap));
+  BP_TRY(sc.get(&a.counters, 6));
+  BP_TRY(get_mask(&a.out, n, sc));
+  int dev = 0, sms = 0;
+  BP_CUDA(cudaGetDevice(&dev));
+  BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // one block per SM: they are resident together, and a barrier of few blocks is
+  // the quicker one
+  const unsigned grid = grid_for(cap, kDistThreads, sms);
+  void* args[] = {&a};
+  BP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(distance_kernel), dim3(grid),
+                                      dim3(kDistThreads), args, 0, st));
+  BP_LAUNCHED("distance_kernel");
+  *out = a.out;
+  return scan_counts(*out, st);
+}
+
 // Peaks of x in SciPy's order of conditions: local maxima (plateaus by their
-// midpoint), height, distance, prominence.  Writes `*m_out` entries of `out`.
+// midpoint), height, threshold, distance, prominence.  Writes `*m_out` entries
+// of `out`.
 int find_peaks_impl(const float* x, int n, const bp_peak_options& o, const PeakOut& out,
                     int* m_out, Scratch& sc, cudaStream_t st) {
   *m_out = 0;
   if (n < 3) return BP_OK;
-  int *flags = nullptr, *rank = nullptr, *plateau = nullptr, *counters = nullptr;
-  BP_TRY(sc.get(&flags, (size_t)n + 1));
-  BP_TRY(sc.get(&rank, (size_t)n + 1));
-  BP_TRY(sc.get(&plateau, n));
-  BP_TRY(sc.get(&counters, 4));
-  BP_CUDA(cudaMemsetAsync(flags, 0, ((size_t)n + 1) * sizeof(int), st));
-  BP_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(int), st));
-  local_max_kernel<<<grid_for(n, 256), 256, 0, st>>>(x, n, flags, plateau, counters);
-  BP_LAUNCHED("local_max_kernel");
-  int n_plateau = 0;
-  BP_TRY(read_back(&n_plateau, counters, st));
-  if (n_plateau > 0) {
-    plateau_kernel<<<grid_for((long long)n_plateau * 32, 256), 256, 0, st>>>(x, n, plateau,
-                                                                             counters, flags);
-    BP_LAUNCHED("plateau_kernel");
+  Mask peaks{};
+  int *pos = nullptr, *flags = nullptr;
+  BP_TRY(local_maxima(x, n, &peaks, sc, st));
+  int cap = n / 2 + 1;  // peaks, at most
+  const int* d_m = peaks.counts + peaks.n_blocks;
+  BP_TRY(sc.get(&pos, cap));
+  positions_kernel<<<(unsigned)peaks.n_blocks, kMaskThreads, 0, st>>>(n, peaks, pos);
+  BP_LAUNCHED("positions_kernel");
+  int m = -1;  // not read back yet
+  if (o.use_height || o.use_threshold || o.use_prominence) {
+    BP_TRY(read_back(&m, d_m, st));
+    BP_TRY(sc.get(&flags, (size_t)m + 1));
+    cap = std::max(m, 1);
   }
-  BP_TRY(scan_flags(flags, rank, n, sc, st));
-  int m = 0;
-  BP_TRY(read_back(&m, rank + n, st));
-  int* pos = nullptr;
-  BP_TRY(sc.get(&pos, std::max(m, 1)));
-  scatter_flagged_kernel<<<grid_for(n, 256), 256, 0, st>>>(flags, rank, n, pos);
-  BP_LAUNCHED("scatter_flagged_kernel");
   // height
   if (o.use_height && m > 0) {
     height_flags_kernel<<<grid_for((long long)m + 1, 256), 256, 0, st>>>(
         x, pos, m, o.height_min, o.height_max, o.d_height_min, o.d_height_max, flags);
     BP_LAUNCHED("height_flags_kernel");
-    BP_TRY(keep_flagged(flags, m, &pos, sc, st, &m));
+    BP_TRY(keep_flagged(flags, m, &pos, sc, st, &m, &d_m));
   }
   // threshold
   if (o.use_threshold && m > 0) {
@@ -725,40 +927,18 @@ int find_peaks_impl(const float* x, int n, const bp_peak_options& o, const PeakO
         x, pos, m, o.threshold_min, o.threshold_max, o.d_threshold_min, o.d_threshold_max,
         flags);
     BP_LAUNCHED("threshold_flags_kernel");
-    BP_TRY(keep_flagged(flags, m, &pos, sc, st, &m));
+    BP_TRY(keep_flagged(flags, m, &pos, sc, st, &m, &d_m));
   }
-  // greedy distance rule, in rounds
-  if (o.distance > 0.0 && m > 1) {
-    const double dc = std::ceil(o.distance);
-    const long long dist = dc > (double)n ? (long long)n + 1 : (long long)dc;
-    float* val = nullptr;
-    int *state = nullptr, *und = nullptr, *und2 = nullptr, *kept = nullptr;
-    BP_TRY(sc.get(&val, m));
-    BP_TRY(sc.get(&state, (size_t)m + 1));
-    BP_TRY(sc.get(&und, m));
-    BP_TRY(sc.get(&und2, m));
-    BP_TRY(sc.get(&kept, m));
-    gather_heights_kernel<<<grid_for(m, 256), 256, 0, st>>>(x, pos, m, val, state, und);
-    BP_LAUNCHED("gather_heights_kernel");
-    int u = m;
-    for (int round = 0; u > 0; ++round) {
-      if (round > m) return fail(BP_ERR_KERNEL, "distance rule did not converge");
-      BP_CUDA(cudaMemsetAsync(counters + 1, 0, 2 * sizeof(int), st));
-      const unsigned gw = grid_for((long long)u * 32, 256);
-      distance_keep_kernel<<<gw, 256, 0, st>>>(pos, val, state, m, dist, und, u, kept,
-                                               counters + 1);
-      BP_LAUNCHED("distance_keep_kernel");
-      distance_drop_kernel<<<gw, 256, 0, st>>>(pos, state, m, dist, kept, counters + 1);
-      BP_LAUNCHED("distance_drop_kernel");
-      distance_next_kernel<<<grid_for(u, 256), 256, 0, st>>>(state, und, u, und2, counters + 2);
-      BP_LAUNCHED("distance_next_kernel");
-      BP_TRY(read_back(&u, counters + 2, st));
-      std::swap(und, und2);
-    }
-    kept_flags_kernel<<<grid_for((long long)m + 1, 256), 256, 0, st>>>(state, m, flags);
-    BP_LAUNCHED("kept_flags_kernel");
-    BP_TRY(keep_flagged(flags, m, &pos, sc, st, &m));
+  // greedy distance rule
+  if (o.distance > 0.0 && m != 0) {
+    Mask kept{};
+    BP_TRY(distance_rule(x, n, pos, d_m, cap, o.distance, nullptr, &kept, sc, st));
+    d_m = kept.counts + kept.n_blocks;
+    positions_kernel<<<(unsigned)kept.n_blocks, kMaskThreads, 0, st>>>(n, kept, pos);
+    BP_LAUNCHED("positions_kernel");
+    m = -1;
   }
+  if (m < 0) BP_TRY(read_back(&m, d_m, st));
   // prominence
   if (o.use_prominence && m > 0) {
     double* prom = nullptr;
@@ -814,14 +994,7 @@ extern "C" {
 
 float bp_pairwise_sum_f32(const float* x, size_t n) {
   if (n == 0 || !x || n > (size_t)INT_MAX) return 0.0f;
-  const PwTree t = pw_tree((int)n);
-  std::vector<float> v(t.n_nodes);
-  for (const int4& lf : t.leaves) {
-    const float* base = x + lf.y;
-    v[lf.x] = pw_leaf([&](int i) { return base[i]; }, lf.z);
-  }
-  for (const int4& nd : t.inner) v[nd.x] = v[nd.y] + v[nd.z];
-  return 0.0f + v[t.root];
+  return 0.0f + pw_host(x, (int)n);
 }
 
 int bp_threshold_dev(const float* d_series, size_t n_samples, size_t sliding_window,
@@ -845,33 +1018,43 @@ int bp_threshold_dev(const float* d_series, size_t n_samples, size_t sliding_win
   const int shift = (int)step;  // int() truncation, as in the notebook
   const int n_win = (n - W) / shift + 1;
   Scratch sc(st);
-  int *zflags = nullptr, *zrank = nullptr;
-  float *nz = nullptr, *filled = nullptr, *stats0 = nullptr;
-  BP_TRY(sc.get(&zflags, (size_t)n + 1));
-  BP_TRY(sc.get(&zrank, (size_t)n + 1));
-  BP_TRY(sc.get(&nz, n));
-  BP_TRY(sc.get(&filled, n));
+  Mask zeros{};
+  float* stats0 = nullptr;
+  BP_TRY(get_mask(&zeros, n, sc));
   BP_TRY(sc.get(&stats0, 2));  // default centre, deviation
-  zero_flags_kernel<<<grid_for((long long)n + 1, 256), 256, 0, st>>>(d_series, n, zflags);
-  BP_LAUNCHED("zero_flags_kernel");
-  BP_TRY(scan_flags(zflags, zrank, n, sc, st));
+  zero_mask_kernel<<<(unsigned)zeros.n_blocks, kMaskThreads, 0, st>>>(d_series, n, zeros);
+  BP_LAUNCHED("zero_mask_kernel");
+  BP_TRY(scan_counts(zeros, st));
   int n_zeros = 0;
-  BP_TRY(read_back(&n_zeros, zrank + n, st));
+  BP_TRY(read_back(&n_zeros, zeros.counts + zeros.n_blocks, st));
   if (d_white_noise && n_white_noise < (size_t)n_zeros)
     return fail(BP_ERR_INVALID_ARGUMENT, "white noise holds %zu values for %d zero samples",
                 n_white_noise, n_zeros);
   const int m = n - n_zeros;
-  gather_nonzero_kernel<<<grid_for(n, 256), 256, 0, st>>>(d_series, n, zrank, nz);
-  BP_LAUNCHED("gather_nonzero_kernel");
+  // without a zero the series is its own non-zero samples, and stays as it is
+  const float *nz = d_series, *filled = d_series;
+  float *nz_mem = nullptr, *filled_mem = nullptr;
+  if (n_zeros > 0) {
+    BP_TRY(sc.get(&nz_mem, n));
+    BP_TRY(sc.get(&filled_mem, n));
+    gather_nonzero_kernel<<<(unsigned)zeros.n_blocks, kMaskThreads, 0, st>>>(d_series, n, zeros,
+                                                                             nz_mem);
+    BP_LAUNCHED("gather_nonzero_kernel");
+    nz = nz_mem;
+    filled = filled_mem;
+  }
   // centre and deviation of the non-zero samples (NaN when there are none)
   if (kind == BP_THRESHOLD_RMS) {
-    if (m > 0) {
-      BP_TRY(pw_mean(nz, 0, m, 1, 0, nullptr, stats0, sc, st));
-      BP_TRY(pw_mean(nz, 0, m, 1, 1, stats0, stats0 + 1, sc, st));
+    if (n_zeros == 0) {
+      // nothing to fill
+    } else if (m > 0) {
+      BP_TRY(pw_mean(nz, 0, m, 1, 0, nullptr, false, stats0, sc, st));
+      BP_TRY(pw_mean(nz, 0, m, 1, 1, stats0, true, stats0 + 1, sc, st));
+    } else {
+      no_stats_kernel<<<1, 32, 0, st>>>(stats0);
+      BP_LAUNCHED("no_stats_kernel");
     }
-    finish_stats_kernel<<<1, 32, 0, st>>>(stats0, m > 0 ? 1 : 0);
-    BP_LAUNCHED("finish_stats_kernel");
-  } else {
+  } else if (n_zeros > 0) {
     BP_TRY(np_median(nz, 0, m, 1, 0, nullptr, stats0, sc, st));
     BP_TRY(np_median(nz, 0, m, 1, 1, stats0, stats0 + 1, sc, st));
   }
@@ -883,32 +1066,25 @@ int bp_threshold_dev(const float* d_series, size_t n_samples, size_t sliding_win
     BP_LAUNCHED("normal_kernel");
     noise = gen;
   }
-  fill_zeros_kernel<<<grid_for(n, 256), 256, 0, st>>>(d_series, n, zrank, noise, stats0,
-                                                       stats0 + 1, filled);
-  BP_LAUNCHED("fill_zeros_kernel");
+  if (n_zeros > 0) {
+    fill_zeros_kernel<<<(unsigned)zeros.n_blocks, kMaskThreads, 0, st>>>(
+        d_series, n, zeros, noise, stats0, stats0 + 1, filled_mem);
+    BP_LAUNCHED("fill_zeros_kernel");
+  }
   // per-window centre and spread
-  float *centre = nullptr, *spread = nullptr, *thr = nullptr, *thr2 = nullptr;
+  float *centre = nullptr, *spread = nullptr;
   BP_TRY(sc.get(&centre, n_win));
   BP_TRY(sc.get(&spread, n_win));
-  BP_TRY(sc.get(&thr, n_win));
-  BP_TRY(sc.get(&thr2, n_win));
   if (kind == BP_THRESHOLD_RMS) {
-    BP_TRY(pw_mean(filled, shift, W, n_win, 0, nullptr, centre, sc, st));
-    BP_TRY(pw_mean(filled, shift, W, n_win, 1, centre, spread, sc, st));
+    BP_TRY(pw_mean(filled, shift, W, n_win, 0, nullptr, false, centre, sc, st));
+    BP_TRY(pw_mean(filled, shift, W, n_win, 1, centre, false, spread, sc, st));
   } else {
     BP_TRY(np_median(filled, shift, W, n_win, 0, nullptr, centre, sc, st));
     BP_TRY(np_median(filled, shift, W, n_win, 1, centre, spread, sc, st));
   }
-  const unsigned gwin = grid_for(n_win, 256);
-  window_threshold_kernel<<<gwin, 256, 0, st>>>(centre, spread, n_win,
-                                                kind == BP_THRESHOLD_RMS ? 1 : 0, num_dev, thr);
-  BP_LAUNCHED("window_threshold_kernel");
-  neighbour_max_kernel<<<gwin, 256, 0, st>>>(thr, n_win, -1, thr2);
-  BP_LAUNCHED("neighbour_max_kernel");
-  neighbour_max_kernel<<<gwin, 256, 0, st>>>(thr2, n_win, +1, thr);
-  BP_LAUNCHED("neighbour_max_kernel");
-  spread_threshold_kernel<<<grid_for(n, 256), 256, 0, st>>>(thr, n_win, n, W, half, shift,
-                                                            d_threshold);
+  const WindowThreshold thr{centre, spread, n_win, kind == BP_THRESHOLD_RMS ? 1 : 0, num_dev};
+  spread_threshold_kernel<<<grid_for(n, 1024), 256, 0, st>>>(thr, n, W, half, shift,
+                                                             d_threshold);
   BP_LAUNCHED("spread_threshold_kernel");
   return BP_OK;
 }
@@ -973,6 +1149,23 @@ int bp_detect_dev(const float* d_beam_max, const int32_t* d_argmax, const float*
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   Scratch sc(st);
   const int n = (int)n_samples;
+  if (n < 3) return BP_OK;
+  if (distance > 0.0) {
+    Mask peaks{}, kept{};
+    int *pos = nullptr, k = 0;
+    BP_TRY(local_maxima(d_beam_max, n, &peaks, sc, st));
+    BP_TRY(sc.get(&pos, (size_t)n / 2 + 1));
+    positions_kernel<<<(unsigned)peaks.n_blocks, kMaskThreads, 0, st>>>(n, peaks, pos);
+    BP_LAUNCHED("positions_kernel");
+    BP_TRY(distance_rule(d_beam_max, n, pos, peaks.counts + peaks.n_blocks, n / 2 + 1, distance,
+                         d_threshold, &kept, sc, st));
+    mask_detections_kernel<<<(unsigned)kept.n_blocks, kMaskThreads, 0, st>>>(
+        n, kept, d_beam_max, d_argmax, d_peaks, d_heights, d_sources);
+    BP_LAUNCHED("mask_detections_kernel");
+    BP_TRY(read_back(&k, kept.counts + kept.n_blocks, st));
+    *n_detections = (size_t)k;
+    return BP_OK;
+  }
   int* peaks = nullptr;
   BP_TRY(sc.get(&peaks, n / 2 + 1));
   int m = 0;
