@@ -201,7 +201,7 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
 }
 
 // Packed FP32 pair add (sm_100 .f32x2); each lane equals __fadd_rn.  Only
-// used where no multiply precedes it, so there is nothing to fuse.
+// used where no packed multiply precedes it, so there is nothing to fuse.
 __device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
   float2 d;
   asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
@@ -213,6 +213,24 @@ __device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+// Packed FP32 pair multiply; each lane equals __fmul_rn.  As a fused multiply-add
+// with -0, which changes no product (not the sign of a zero one either): a packed
+// multiply is fused with the packed add that takes it, which would change the last
+// bit.  neg0: -0 in a form that the compiler cannot see through, see neg_zero().
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b, float neg0) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\t"
+      "mov.b64 rb, {%4, %5};\n\t"
+      "mov.b64 rc, {%6, %6};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\t"
+      "mov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(neg0));
+  return d;
+}
+// Grids of these kernels have no z dimension: 1 << 31.
+__device__ __forceinline__ float neg_zero() { return __uint_as_float(gridDim.z << 31); }
 
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

@@ -609,13 +609,10 @@ struct Tm {
 #pragma unroll
       for (int x = 0; x < 8; ++x) acc[x] = add2_rn(acc[x], make_float2(u(2 * x), u(2 * x + 1)));
     } else {
-      // scalar rounded multiply, then rounded add (a packed pair could be
-      // fused downstream, which would change the last bit)
+      const float2 w2 = make_float2(w, w);  // rounded multiply, then rounded add
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        acc[x].x = __fadd_rn(acc[x].x, __fmul_rn(w, u(2 * x)));
-        acc[x].y = __fadd_rn(acc[x].y, __fmul_rn(w, u(2 * x + 1)));
-      }
+      for (int x = 0; x < 8; ++x)
+        acc[x] = add2_rn(acc[x], mul2_rn(w2, make_float2(u(2 * x), u(2 * x + 1)), neg_zero()));
     }
   }
 
