@@ -130,6 +130,9 @@ struct bp_table {
   int* status;       // kernel status word
   double mean_spread;  // mean span of the used (tile, station, phase) windows
   bool real_weights;   // some weight is neither 0 nor 1
+  // Tiles in ascending order of their widest window (of tables with windows too
+  // wide for the tensor-memory kernel; empty otherwise): its span, and the mean.
+  std::vector<int> tile_max, tile_mean;
   int device;
   cudaStream_t stream;
 };
@@ -148,6 +151,13 @@ __global__ void init_stats_kernel(int* stats, int* status) {
     for (int i = 7; i < bp::kStatCount; ++i) stats[i] = 0;
     *status = 0;
   }
+}
+
+// Tile i of `to` is tile order[i] of `from` (64 threads per tile).
+__global__ void permute_tiles_kernel(const int* __restrict__ from, const int* __restrict__ order,
+                                     int* __restrict__ to) {
+  to[blockIdx.x * bp::kTableTile + threadIdx.x] =
+      from[order[blockIdx.x] * bp::kTableTile + threadIdx.x];
 }
 
 template <int P>
@@ -238,6 +248,57 @@ int build_tiling_map(const int32_t* d_delays, const float* d_w, size_t N, size_t
   if (e != cudaSuccess) rc = cuda_fail(e, "tiling map");
   if (scratch) cudaFreeAsync(scratch, st);
   return rc;
+}
+
+int build_tiles(const int32_t* d_delays, const float* d_w, bp::TableDev& tb, cudaStream_t st) {
+  switch (tb.P) {
+    case 1: return launch_table_build<1>(d_delays, d_w, tb, st);
+    case 2: return launch_table_build<2>(d_delays, d_w, tb, st);
+    case 3: return launch_table_build<3>(d_delays, d_w, tb, st);
+    case 4: return launch_table_build<4>(d_delays, d_w, tb, st);
+  }
+  return BP_OK;
+}
+
+// Puts a built table's tiles in ascending order of their widest window and
+// builds them again; their widest and mean spans stay on the host.
+int order_tiles(bp_table* t, const int32_t* d_delays, const float* d_w, cudaStream_t st) {
+  const int n = t->dev.n_tiles;
+  std::vector<int2> hdr(n);
+  BP_CUDA(cudaMemcpyAsync(hdr.data(), t->dev.tile_hdr, n * sizeof(int2), cudaMemcpyDeviceToHost,
+                          st));
+  BP_CUDA(cudaStreamSynchronize(st));
+  std::vector<int> order(n);
+  for (int i = 0; i < n; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return (hdr[a].y & 0xFFFF) < (hdr[b].y & 0xFFFF); });
+  char* scratch = nullptr;
+  const size_t o_perm = pad256((size_t)n * sizeof(int)),
+               perm_bytes = (size_t)n * bp::kTableTile * sizeof(int);
+  BP_CUDA(cudaMallocAsync(&scratch, o_perm + perm_bytes, st));
+  int* d_order = reinterpret_cast<int*>(scratch);
+  int* d_perm = reinterpret_cast<int*>(scratch + o_perm);
+  cudaError_t e = cudaMemcpyAsync(d_order, order.data(), n * sizeof(int), cudaMemcpyHostToDevice,
+                                  st);
+  if (e == cudaSuccess) {
+    permute_tiles_kernel<<<(unsigned)n, bp::kTableTile, 0, st>>>(t->dev.perm, d_order, d_perm);
+    g_launches.fetch_add(1);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(const_cast<int*>(t->dev.perm), d_perm, perm_bytes,
+                        cudaMemcpyDeviceToDevice, st);
+  cudaFreeAsync(scratch, st);
+  if (e != cudaSuccess) return cuda_fail(e, "order of the tiles");
+  if (int rc = build_tiles(d_delays, d_w, t->dev, st)) return rc;
+  // `order` is pageable: its copy has left it before the call returned
+  t->tile_max.resize(n);
+  t->tile_mean.resize(n);
+  for (int i = 0; i < n; ++i) {
+    t->tile_max[i] = hdr[order[i]].y & 0xFFFF;
+    t->tile_mean[i] = (int)((unsigned)hdr[order[i]].y >> 16);
+  }
+  return BP_OK;
 }
 
 template <bool MAXRED>
@@ -371,10 +432,13 @@ struct PlanesScratch {
   }
 };
 
-int rowcap_for(const bp_table* t, int cfg) {
-  if (cfg == kTmemConfig)
-    return bp::tm_rows(t->info.max_spread + 15);  // plane rows
-  return (int)bp::align_up_sz((size_t)(cfg_time_tile(cfg) + t->info.max_spread + 1),
+// The widest window that a launch on table `t` has: the table's, or `spread`
+// when it takes some of its tiles.
+int spread_of(const bp_table* t, int spread) { return spread >= 0 ? spread : t->info.max_spread; }
+
+int rowcap_for(const bp_table* t, int cfg, int spread = -1) {
+  if (cfg == kTmemConfig) return bp::tm_rows(spread_of(t, spread) + 15);  // plane rows
+  return (int)bp::align_up_sz((size_t)(cfg_time_tile(cfg) + spread_of(t, spread) + 1),
                               bp::kAlign);
 }
 
@@ -393,14 +457,14 @@ int device_smem_per_sm(int dev) {
 // SM (a two-block shape left at one block per SM runs at half its
 // occupancy).  Without the max reduction the buffer is empty.
 // The tensor-memory kernel: its ring stages in the place of the rows.
-int rows_for(const bp_table* t, int c, int storage, bool maxred) {
+int rows_for(const bp_table* t, int c, int storage, bool maxred, int spread = -1) {
   if (c == kTmemConfig)
-    return tmem_stages(t->dev.S, t->dev.P, maxred, t->info.max_spread,
+    return tmem_stages(t->dev.S, t->dev.P, maxred, spread_of(t, spread),
                        std::max(1, t->info.max_active), storage, t->device);
   const int ws = cfg_of(c).ws;
   const int minb = cfg_of(c).minb;
   for (int rows : {ws, 1}) {
-    const size_t need = staged_smem_bytes(c, t->dev.P, maxred, rowcap_for(t, c),
+    const size_t need = staged_smem_bytes(c, t->dev.P, maxred, rowcap_for(t, c, spread),
                                           std::max(1, t->info.max_active), storage, rows);
     if (need <= (size_t)device_smem_optin(t->device) &&
         (need + 1024) * (size_t)minb <= (size_t)device_smem_per_sm(t->device))
@@ -410,8 +474,8 @@ int rows_for(const bp_table* t, int c, int storage, bool maxred) {
   return 0;
 }
 
-bool config_fits(const bp_table* t, int c, int storage, bool maxred) {
-  return rows_for(t, c, storage, maxred) > 0;
+bool config_fits(const bp_table* t, int c, int storage, bool maxred, int spread = -1) {
+  return rows_for(t, c, storage, maxred, spread) > 0;
 }
 
 // Fallback order when the chosen shape does not fit a table, fastest first
@@ -433,12 +497,15 @@ const int kOrder16[kStagedConfigs] = {2, 1, 6, 7, 0, 5, 4, 3, 8};
 //   3 phases, max, 0 / 1: 50: 4.03 | 2.88, 89: 3.45 | 3.61
 // 16-bit storage halves what the staged shapes read and keeps them ahead
 // (FP16, span 65: 1.47 | 2.27).
-bool prefers_tmem(const bp_table* t, int storage, bool maxred) {
-  if (storage != BP_STORAGE_F32) return false;
+double tmem_limit(const bp_table* t, int storage, bool maxred) {
+  if (storage != BP_STORAGE_F32) return -1.0;
   double limit = t->real_weights ? 90.0 : 145.0;
   if (t->dev.P > 2) limit = std::min(limit, 80.0);
   if (!maxred) limit -= 30.0;
-  return t->mean_spread <= limit;
+  return limit;
+}
+bool prefers_tmem(const bp_table* t, int storage, bool maxred) {
+  return t->mean_spread <= tmem_limit(t, storage, maxred);
 }
 
 // The caller's choice if it serves this table; else the tensor-memory kernel
@@ -457,6 +524,67 @@ int config_for(const bp_table* t, int storage, bool maxred, bool staged_only = f
   for (int i = 0; i < kStagedConfigs; ++i)
     if (config_fits(t, order[i], storage, maxred)) return order[i];
   return 0;
+}
+
+// Tiles [tile0, tile0 + n_tiles) of a table, which one launch takes.
+struct Part {
+  int cfg, tile0, n_tiles, spread;
+};
+
+// The launches of a plain call on table `t` (n_tt: its 512-sample time tiles).
+// One, unless some tiles' windows are too wide for the kernel that is the fastest
+// for the others: a few wide tiles (sources at a grid's edge or near a station)
+// would otherwise decide for all of them.  The first part is what the
+// tensor-memory kernel is the faster one for, the next the tiles that the first
+// staged shape serves which serves half of what is left, then the widest.  Every
+// launch ends in a partly filled wave of blocks, so a part has at least 32 tile
+// pairs (sources x time) per SM, else it goes with the next wider one.
+// (16,000 sources, 60 stations, 60,007 samples, windows of up to 4,300 samples,
+// weights not 0 / 1: 18.5 ms as one launch, 15.8 ms as two.)
+std::vector<Part> parts_of(const bp_table* t, int storage, bool maxred, bool staged_only,
+                           long long n_tt) {
+  const int n = t->dev.n_tiles;
+  std::vector<Part> parts;
+  const int c = chosen_config(storage, maxred);
+  const bool chosen =
+      c >= 0 && !(staged_only && c == kTmemConfig) && config_fits(t, c, storage, maxred);
+  int at = 0;
+  if (!chosen && (int)t->tile_max.size() == n) {
+    const long long least = 32ll * std::max(1, device_sm_count(t->device));
+    auto fit = [&](int cfg) {  // tiles that a config serves: a prefix
+      int lo = 0, hi = n;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (config_fits(t, cfg, storage, maxred, t->tile_max[mid - 1])) lo = mid;
+        else hi = mid - 1;
+      }
+      return lo;
+    };
+    auto add = [&](int cfg, int end) {
+      if ((long long)(end - at) * n_tt < least) return;
+      parts.push_back(Part{cfg, at, end - at, t->tile_max[end - 1]});
+      at = end;
+    };
+    if (!staged_only) {
+      const double limit = tmem_limit(t, storage, maxred);
+      int narrow = 0;
+      for (int i = 0; i < n; ++i) narrow += t->tile_mean[i] <= limit;
+      add(kTmemConfig, std::min(narrow, fit(kTmemConfig)));
+    }
+    const int* order = storage == BP_STORAGE_F32 ? kOrderF32 : kOrder16;
+    for (int i = 0; at < n && i < kStagedConfigs; ++i) {
+      const int end = fit(order[i]);
+      if (end - at < (n - at + 1) / 2) continue;
+      if (end < n) add(order[i], end);
+      break;
+    }
+  }
+  if (at < n) {
+    const int cfg = at == 0 ? config_for(t, storage, maxred, staged_only)
+                            : config_for(t, storage, maxred, true);
+    parts.push_back(Part{cfg, at, n - at, t->info.max_spread});
+  }
+  return parts;
 }
 
 // Rows of the max buffer, or the tensor-memory kernel's ring stages.
@@ -496,24 +624,67 @@ int check_layout(const bp_table* t, size_t n_samples, size_t lpad, size_t pitch)
   return BP_OK;
 }
 
-bp::TableView table_view(const bp_table* t) {
+// A table's tiles from tile0 on (n_tiles of them; -1: all).
+bp::TableView table_view(const bp_table* t, int tile0 = 0, int n_tiles = -1) {
+  const size_t SP = (size_t)t->dev.S * t->dev.P;
+  const size_t meta_elem = t->dev.P <= 2 ? sizeof(uint2) : sizeof(uint4);
   bp::TableView v{};
-  v.src_info = t->dev.src_info;
-  v.tile_hdr = t->dev.tile_hdr;
-  v.st_s = t->dev.st_s;
-  v.st_lo = t->dev.st_lo;
-  v.st_spread = t->dev.st_spread;
-  v.meta = t->dev.meta;
+  v.src_info = t->dev.src_info + (size_t)tile0 * t->dev.K;
+  v.tile_hdr = t->dev.tile_hdr + tile0;
+  v.st_s = t->dev.st_s + (size_t)tile0 * t->dev.S;
+  v.st_lo = t->dev.st_lo + tile0 * SP;
+  v.st_spread = t->dev.st_spread + tile0 * SP;
+  v.meta = static_cast<const char*>(t->dev.meta) +
+           (size_t)tile0 * t->dev.S * t->dev.K * meta_elem;
   v.S = t->dev.S;
-  v.n_tiles = t->dev.n_tiles;
+  v.n_tiles = n_tiles >= 0 ? n_tiles : t->dev.n_tiles;
   return v;
+}
+
+// The launches of a plain call: a.rec0 is its record (planes not set).
+int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bool checked,
+              cudaStream_t st) {
+  bp::RecordView& r = a.rec0;
+  const int whole = 32 * 16;
+  const long long n_tt = (r.out1 + whole - 1) / whole - r.out0 / whole;
+  std::vector<Part> parts = parts_of(t, storage, maxred, checked, n_tt);
+  PlanesScratch planes;
+  if (n_tt > 0 && !parts.empty() && parts[0].cfg == kTmemConfig) {
+    const size_t pitch = (size_t)r.pitch;
+    if (planes.get(planes_bytes(t->dev.S, t->dev.P, pitch), st)) {
+      if (int rc = fill_planes(t->dev.S, t->dev.P, storage, r.traces, pitch, planes.p, st))
+        return rc;
+      r.planes = static_cast<const unsigned char*>(planes.p);
+    } else {
+      parts = parts_of(t, storage, maxred, true, n_tt);
+    }
+  }
+  a.max_active = std::max(1, t->info.max_active);
+  a.status = t->status;
+  for (const Part& p : parts) {
+    const int tt = cfg_time_tile(p.cfg);
+    const int n_tau = (r.out1 + tt - 1) / tt - r.out0 / tt;
+    if (n_tau <= 0) return BP_OK;
+    a.tab0 = table_view(t, p.tile0, p.n_tiles);
+    const int n_btiles = p.n_tiles * cfg_blocks_per_tile(p.cfg);
+    a.tiles_per_chunk = choose_tiles_per_chunk(n_tau, n_btiles, t->device);
+    a.rowcap = rowcap_for(t, p.cfg, p.spread);
+    set_fit(a, p.cfg, rows_for(t, p.cfg, storage, maxred, p.spread));
+    const long long blocks =
+        (long long)((n_tau + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
+    const int rc = maxred ? launch_window<true>(p.cfg, t->dev.P, checked, storage, a, false,
+                                                blocks, t->device, st)
+                          : launch_window<false>(p.cfg, t->dev.P, checked, storage, a, false,
+                                                 blocks, t->device, st);
+    if (rc) return rc;
+  }
+  return BP_OK;
 }
 
 int run_staged(const bp_table* t, const void* traces, int storage, const float* scales,
                size_t T, size_t lpad, size_t pitch, int out_of_bounds, unsigned long long* keys,
                float* beam, size_t ldb, cudaStream_t st) {
   bp::LaunchArgs a{};
-  a.tab0 = table_view(t);
   bp::RecordView& r = a.rec0;
   r.traces = traces;
   r.scales = scales;
@@ -528,32 +699,7 @@ int run_staged(const bp_table* t, const void* traces, int storage, const float* 
   r.beam = beam;
   r.ldb = (long long)ldb;
   const bool maxred = keys != nullptr;
-  const bool checked = out_of_bounds && t->info.any_nonfinite;
-  int cfg = config_for(t, storage, maxred, checked);
-  PlanesScratch planes;
-  if (cfg == kTmemConfig && T > 0) {
-    if (planes.get(planes_bytes(t->dev.S, t->dev.P, pitch), st)) {
-      if (int rc = fill_planes(t->dev.S, t->dev.P, storage, traces, pitch, planes.p, st))
-        return rc;
-      r.planes = static_cast<const unsigned char*>(planes.p);
-    } else {
-      cfg = config_for(t, storage, maxred, true);
-    }
-  }
-  const int tt = cfg_time_tile(cfg);
-  const int n_tt = (int)((T + tt - 1) / tt);
-  const int n_btiles = t->dev.n_tiles * cfg_blocks_per_tile(cfg);
-  a.tiles_per_chunk = choose_tiles_per_chunk(n_tt, n_btiles, t->device);
-  a.rowcap = rowcap_for(t, cfg);
-  a.max_active = std::max(1, t->info.max_active);
-  set_fit(a, cfg, rows_for(t, cfg, storage, maxred));
-  a.status = t->status;
-  if (n_tt == 0) return BP_OK;
-  const long long blocks =
-      (long long)((n_tt + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
-  if (maxred)
-    return launch_window<true>(cfg, t->dev.P, checked, storage, a, false, blocks, t->device, st);
-  return launch_window<false>(cfg, t->dev.P, checked, storage, a, false, blocks, t->device, st);
+  return run_parts(t, a, storage, maxred, out_of_bounds && t->info.any_nonfinite, st);
 }
 
 int run_direct(const void* traces, int storage, const float* scales, size_t T, size_t lpad,
@@ -792,12 +938,7 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
     g_launches.fetch_add(1);
     if (cudaError_t le = cudaGetLastError(); le != cudaSuccess)
       return bail(cuda_fail(le, "launch sort_tile_slots_kernel"));
-    switch (P) {
-      case 1: rc = launch_table_build<1>(d_delays, d_weights, t->dev, st); break;
-      case 2: rc = launch_table_build<2>(d_delays, d_weights, t->dev, st); break;
-      case 3: rc = launch_table_build<3>(d_delays, d_weights, t->dev, st); break;
-      case 4: rc = launch_table_build<4>(d_delays, d_weights, t->dev, st); break;
-    }
+    rc = build_tiles(d_delays, d_weights, t->dev, st);
     if (rc) return bail(rc);
   }
   int stats[bp::kStatCount];
@@ -830,6 +971,10 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
   in.uses_window_kernel = window && n_tiles > 0 && !stats[bp::kStatWideTile] ? 1 : 0;
   if (in.uses_window_kernel && !staged_serves(t, BP_STORAGE_F32, true)) in.uses_window_kernel = 0;
   const bool use_window = in.uses_window_kernel != 0;
+  // windows that the tensor-memory kernel does not take: tiles by width, for
+  // parts_of
+  if (use_window && n_tiles > 1 && !config_fits(t, kTmemConfig, BP_STORAGE_F32, true))
+    if (int rc2 = order_tiles(t, d_delays, d_weights, st)) return bail(rc2);
   if (!use_window && N > 0) {
     // The direct kernel reads the raw arrays: keep private copies.
     e = cudaMallocAsync(&t->direct_mem, N * S * P * sizeof(int32_t) + N * S * sizeof(float) + 256,
@@ -1774,7 +1919,6 @@ int bp_record_beamform_max_dev(const bp_table* t, const bp_record* q, int storag
     storage = BP_STORAGE_F32;
   }
   bp::LaunchArgs a{};
-  a.tab0 = table_view(t);
   bp::RecordView& r = a.rec0;
   r.traces = expand ? static_cast<const void*>(f32.p) : q->traces;
   r.scales = expand ? nullptr : q->scales;
@@ -1787,31 +1931,7 @@ int bp_record_beamform_max_dev(const bp_table* t, const bp_record* q, int storag
   r.flexible = q->out_of_bounds;
   r.keys = keys;
   const bool checked = q->out_of_bounds && t->info.any_nonfinite;
-  int cfg = config_for(t, storage, true, checked);
-  PlanesScratch planes;
-  if (cfg == kTmemConfig) {
-    if (planes.get(planes_bytes(t->dev.S, t->dev.P, q->pitch), st)) {
-      if (int rc = fill_planes(t->dev.S, t->dev.P, storage, r.traces, q->pitch, planes.p, st))
-        return rc;
-      r.planes = static_cast<const unsigned char*>(planes.p);
-    } else {
-      cfg = config_for(t, storage, true, true);
-    }
-  }
-  const int tt = cfg_time_tile(cfg);
-  const int tau_first = r.out0 / tt;
-  const int n_tt = (r.out1 + tt - 1) / tt - tau_first;
-  const int n_btiles = t->dev.n_tiles * cfg_blocks_per_tile(cfg);
-  a.tiles_per_chunk = choose_tiles_per_chunk(n_tt, n_btiles, t->device);
-  a.rowcap = rowcap_for(t, cfg);
-  a.max_active = std::max(1, t->info.max_active);
-  set_fit(a, cfg, rows_for(t, cfg, storage, true));
-  a.status = t->status;
-  const long long blocks =
-      (long long)((n_tt + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
-  if (int rc = launch_window<true>(cfg, t->dev.P, checked, storage, a, false, blocks, t->device,
-                                   st))
-    return rc;
+  if (int rc = run_parts(t, a, storage, true, checked, st)) return rc;
   bp::decode_keys_kernel<<<(unsigned)((n_out + 255) / 256), 256, 0, st>>>(
       keys, (int)n_out, q->beam_max, q->argmax);
   BP_LAUNCHED("decode_keys_kernel");

@@ -56,7 +56,7 @@ constexpr int kMaxTimeTile = 1024;
 struct TableDev {
   int N, S, P, K, n_tiles;
   int4* src_info;    // [n_tiles * K]  {source index or -1, min delay, max delay, 0}
-  int2* tile_hdr;    // [n_tiles]      {active stations, 0}
+  int2* tile_hdr;    // [n_tiles]      {active stations, mean span << 16 | widest}
   int* st_s;         // [n_tiles * S]  station of active slot j
   int* st_lo;        // [n_tiles * S * P] window start (aligned)
   int* st_spread;    // [n_tiles * S * P] window span beyond the time tile
@@ -204,7 +204,9 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
     for (int o = 16; o > 0; o >>= 1) spread_sum += __shfl_xor_sync(0xFFFFFFFFu, spread_sum, o);
     if (lane == 0) {
       n_active_sh = n;
-      tb.tile_hdr[tile] = make_int2(n, 0);
+      const unsigned mean = n ? (unsigned)(spread_sum / (unsigned)(n * P)) : 0u;
+      tb.tile_hdr[tile] =
+          make_int2(n, (int)(min(mean, 0xFFFFu) << 16 | min((unsigned)spread_max, 0xFFFFu)));
       if (n > 0) {
         atomicMin(&tb.stats[kStatMinDelay], mn);
         atomicMax(&tb.stats[kStatMaxDelay], mx);
@@ -275,7 +277,7 @@ __global__ void table_build_kernel(const int32_t* __restrict__ delays,
 // A travel-time table as the staged kernel reads it.
 struct TableView {
   const int4* src_info;  // [n_tiles * K] {source index or -1, min delay, max delay, 0}
-  const int2* tile_hdr;  // [n_tiles] {active stations, 0}
+  const int2* tile_hdr;  // [n_tiles] {active stations, mean span << 16 | widest}
   const int* st_s;       // [n_tiles * S]
   const int* st_lo;      // [n_tiles * S * P]
   const int* st_spread;  // [n_tiles * S * P]
