@@ -1,9 +1,10 @@
-"""Autotuner of the staged kernel's shape.
+"""Autotuner of the beam kernel's shape.
 
 The library compiles the staged kernel in several shapes (sources per
 thread, samples per lane, consumer warps, ring stages, stations per ring
 stage, sources per block; see ``bp_kernel_config_describe`` and
-``bp_kernel_config_shape``), all over the same 64-source tables.  Which is
+``bp_kernel_config_shape``) and the tensor-memory kernel as the last config,
+all over the same 64-source tables.  Which is
 fastest depends on the storage type (FP32 is shared-memory bound, 16-bit
 storage issue bound), the number of phases and the tables' delay spread.
 ``autotune`` times every shape on the caller's own table and traces, keeps

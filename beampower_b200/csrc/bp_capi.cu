@@ -641,6 +641,10 @@ bp::TableView table_view(const bp_table* t, int tile0 = 0, int n_tiles = -1) {
   return v;
 }
 
+// Up to this many (table tile, time tile) pairs per SM the tensor-memory kernel's
+// blocks take equal shares of them (see beam_tmem_share_kernel).
+constexpr long long kSharePairs = 16;
+
 // The launches of a plain call: a.rec0 is its record (planes not set).
 int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bool checked,
               cudaStream_t st) {
@@ -670,8 +674,13 @@ int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bo
     a.tiles_per_chunk = choose_tiles_per_chunk(n_tau, n_btiles, t->device);
     a.rowcap = rowcap_for(t, p.cfg, p.spread);
     set_fit(a, p.cfg, rows_for(t, p.cfg, storage, maxred, p.spread));
-    const long long blocks =
+    long long blocks =
         (long long)((n_tau + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
+    const int sms = std::max(1, device_sm_count(t->device));
+    if (p.cfg == kTmemConfig && (long long)n_tau * n_btiles <= kSharePairs * sms) {
+      a.tiles_per_chunk = 0;
+      blocks = std::min<long long>((long long)n_tau * n_btiles, sms);
+    }
     const int rc = maxred ? launch_window<true>(p.cfg, t->dev.P, checked, storage, a, false,
                                                 blocks, t->device, st)
                           : launch_window<false>(p.cfg, t->dev.P, checked, storage, a, false,

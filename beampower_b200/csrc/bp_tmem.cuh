@@ -959,6 +959,66 @@ beam_tmem_kernel(const __grid_constant__ LaunchArgs a) {
   }
 }
 
+// Plain launch of few (table tile, time tile) pairs per SM: a block per SM, and
+// each takes an equal share of the pairs, tile after tile.  No last wave that is
+// partly filled, and one prologue and TMEM allocation for a tile's pairs (4,000
+// sources, 20 stations, 6,000 samples, five pairs per SM: 157 us with a block per
+// pair, 130 us with shares).  With many pairs blocks of a few are the better
+// balance, since tiles differ in cost (52,311 sources, 37 stations, 15,001
+// samples, 166 pairs per SM: 5.3 ms, and 6.8 ms with shares), and the loop over a
+// share costs them registers (2% in beam_tmem_kernel).
+struct TmItem {
+  int tile, tau0, tau1;
+};
+// The block's item that starts `done` time tiles into its share; empty behind
+// the last one.
+__device__ __forceinline__ TmItem tm_item(const LaunchArgs& a, int done) {
+  const int first = a.rec0.out0 / kTmTile;
+  const int n_tau = (a.rec0.out1 + kTmTile - 1) / kTmTile - first;
+  const long long pairs = (long long)a.tab0.n_tiles * n_tau;
+  const long long j = pairs * blockIdx.x / gridDim.x + done;
+  const long long end = pairs * (blockIdx.x + 1) / gridDim.x;
+  const int tile = (int)(j / n_tau), from = (int)(j - (long long)tile * n_tau);
+  return TmItem{tile, first + from, first + from + (int)min(end - j, (long long)(n_tau - from))};
+}
+
+template <int P, bool MAXRED, int STORAGE>
+__global__ void __launch_bounds__(kTmThreads, 1)
+beam_tmem_share_kernel(const __grid_constant__ LaunchArgs a) {
+  using T = Tm<P, MAXRED, STORAGE>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const typename T::Smem sm{smem, a.tm};
+  T::start(sm);
+  typename T::State st;
+  int done = 0;
+  TmItem it = tm_item(a, 0);
+  bool fast16 = T::prologue(sm, a.tab0, a.rec0, it.tile, it.tau0, it.tau1, a.rowcap, a.status);
+  // To the next item; false behind the last one.
+  auto next = [&]() {
+    done += it.tau1 - it.tau0;
+    __syncthreads();
+    it = tm_item(a, done);
+    if (it.tau0 >= it.tau1 || *sm.abort_flag()) return false;
+    fast16 = T::prologue(sm, a.tab0, a.rec0, it.tile, it.tau0, it.tau1, a.rowcap, a.status);
+    return true;
+  };
+  if ((threadIdx.x >> 5) < kTmCompute) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    do {
+      T::compute_item(sm, a.rec0, it.tau0, it.tau1, fast16, a.status, st);
+    } while (next());
+    tm_fence_before();
+    __syncthreads();
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    do {
+      T::produce(sm, it.tau0, it.tau1, a.status, st);
+    } while (next());
+    T::drain(sm, (threadIdx.x >> 5) - kTmCompute, st);
+    T::finish(sm);
+  }
+}
+
 // Persistent launch over a batch's work queue (see beam_batch_kernel).
 template <int P, int STORAGE>
 __global__ void __launch_bounds__(kTmThreads, 1)

@@ -27,13 +27,15 @@ int launch_tmem_p(bp::LaunchArgs a, bool batch, long long plain_blocks, int dev,
     }
     return BP_OK;
   }
-  auto kern = bp::beam_tmem_kernel<P, MAXRED, STORAGE>;
+  const bool share = a.tiles_per_chunk == 0;  // a block per SM, equal shares
+  auto kern = share ? bp::beam_tmem_share_kernel<P, MAXRED, STORAGE>
+                    : bp::beam_tmem_kernel<P, MAXRED, STORAGE>;
   BP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)lay.total));
   if (plain_blocks > kMaxInt) return fail(BP_ERR_UNSUPPORTED, "grid too large");
   if (plain_blocks <= 0) return BP_OK;
   kern<<<(unsigned)plain_blocks, bp::kTmThreads, lay.total, st>>>(a);
-  BP_LAUNCHED("beam_tmem_kernel");
+  BP_LAUNCHED("tensor-memory kernel");
   return BP_OK;
 }
 

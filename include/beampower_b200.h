@@ -464,7 +464,8 @@ BP_API int bp_set_kernel_config(int storage, int reduce, int config);
 BP_API int bp_get_kernel_config(int storage, int reduce);
 /* The shape a call on this table runs with (storage, reduce): the chosen one
  * when its shared memory and blocks per SM fit the table, else the first
- * that fits in a fixed, measured order; -1 when no shape holds the table's
+ * that fits in a fixed, measured order (of a table whose tiles run as several
+ * launches, without a chosen shape: the widest tiles'); -1 when no shape holds the table's
  * windows in this storage (16-bit calls then expand their traces to FP32 and
  * run the FP32 shape, with the direct kernel's values, when that fits; else,
  * and for tables with uses_window_kernel == 0, the direct kernel runs); a
