@@ -1624,6 +1624,27 @@ __global__ void split_keys_kernel(const int32_t* __restrict__ delays, int D, int
   keys[pos] = ((unsigned long long)(uint32_t)g << 32) | low;
 }
 
+// Warp-wide sum / or / and / lanes with the same value.  (The host-side layout
+// check compiles this header for nvcc's default architecture, which has none of
+// them and runs no kernel.)
+#if !defined(__CUDA_ARCH__) || __CUDA_ARCH__ >= 800
+__device__ __forceinline__ int warp_add(int v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
+__device__ __forceinline__ unsigned warp_or(unsigned v) {
+  return __reduce_or_sync(0xFFFFFFFFu, v);
+}
+__device__ __forceinline__ unsigned warp_and(unsigned v) {
+  return __reduce_and_sync(0xFFFFFFFFu, v);
+}
+__device__ __forceinline__ unsigned warp_peers(int v) {
+  return __match_any_sync(0xFFFFFFFFu, v);
+}
+#else
+__device__ __forceinline__ int warp_add(int v) { return v; }
+__device__ __forceinline__ unsigned warp_or(unsigned v) { return v; }
+__device__ __forceinline__ unsigned warp_and(unsigned v) { return v; }
+__device__ __forceinline__ unsigned warp_peers(int v) { return (unsigned)v; }
+#endif
+
 // Shared memory of split_block_kernel.
 constexpr int kMapParts = kMapBlock / kTableTile;
 struct MapBlock {
@@ -1680,7 +1701,7 @@ split_block_kernel(const int32_t* __restrict__ delays, const float* __restrict__
     if (lane == 0) m.warp_sum[warp] = sum;
     __syncthreads();
     int from = lane < warp ? m.warp_sum[lane] : 0;
-    from = __reduce_add_sync(0xFFFFFFFFu, from);
+    from = warp_add(from);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) out[r] += from;
     __syncthreads();
@@ -1740,18 +1761,18 @@ split_block_kernel(const int32_t* __restrict__ delays, const float* __restrict__
         any_set |= u[r];
         all_set &= u[r];
       }
-      peers[r] = __match_any_sync(0xFFFFFFFFu, part[r]);
+      peers[r] = warp_peers(part[r]);
     }
     // The bits that differ between any two delays: those above are common.
-    any_set = __reduce_or_sync(0xFFFFFFFFu, any_set);
-    all_set = __reduce_and_sync(0xFFFFFFFFu, all_set);
+    any_set = warp_or(any_set);
+    all_set = warp_and(all_set);
     if (lane == 0) {
       m.best[warp] = (int)any_set;
       m.warp_sum[warp] = (int)all_set;
     }
     __syncthreads();
-    any_set = __reduce_or_sync(0xFFFFFFFFu, (unsigned)m.best[lane]);
-    all_set = __reduce_and_sync(0xFFFFFFFFu, (unsigned)m.warp_sum[lane]);
+    any_set = warp_or((unsigned)m.best[lane]);
+    all_set = warp_and((unsigned)m.warp_sum[lane]);
     __syncthreads();
     const uint32_t differ = any_set ^ all_set;
     const int bits = 32 - __clz((int)differ);
