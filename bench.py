@@ -526,7 +526,8 @@ def run_ours(args, rank, world, local_rank):
             kms = e0.elapsed_time(e1) / 2
             variants[stg] = {"kernel_ms": kms, "value": terms / (kms * 1e-3),
                              "unit": "beam terms/s", "kernel_config":
-                             lib.bp_get_kernel_config({"fp32": 0, "bf16": 1, "fp16": 2}[stg], 1)}
+                             lib.bp_table_kernel_config(
+                                 vt.handle, {"fp32": 0, "bf16": 1, "fp16": 2}[stg], 1)}
             del tr
         # the other runs of the same configuration: the flexible rule, and
         # reduce='none' on the first 20,000 sources (a 20,000 x T beam)
@@ -643,7 +644,9 @@ def run_ours(args, rank, world, local_rank):
                 "frac": smem_achieved / smem_gbs.value,
                 "traffic": traffic,
                 "note": "shared-memory operand roof (4 B of trace per effective term), peak "
-                        "measured live by bp_measure_peaks; FP32 and HBM views below",
+                        "measured live by bp_measure_peaks; above 1 where the operands "
+                        "come from tensor memory (kernel config 9), whose own roof is 136 "
+                        "words per clock and SM; FP32 and HBM views below",
                 "fp32_view": {"achieved_tflops": eff * 2 / (kernel_ms * 1e-3) / 1e12,
                               "peak_tflops": fp32_tf.value},
                 "hbm_view": {"achieved_gbs": hbm_bytes / (ms_per_step * 1e-3) / 1e9,
