@@ -647,10 +647,15 @@ struct Tm {
     }
   }
 
-  // Fill n, waited for.
-  __device__ static __forceinline__ void tm_take(const Smem& sm, int n, int* status) {
-    mbar_wait_spin(smem_addr(sm.tfull(0)) + (n & 3) * 8, (n >> 2) & 1, sm.abort_flag(), status);
-    __syncwarp();
+  // Fill n, waited for (unless every lane has seen it complete: lanes may see it at
+  // different tries, and the loads that follow are the whole warp's).
+  __device__ static __forceinline__ void tm_take(const Smem& sm, int n, int* status,
+                                                 bool seen = false) {
+    if (!__all_sync(0xFFFFFFFFu, seen)) {
+      mbar_wait_spin(smem_addr(sm.tfull(0)) + (n & 3) * 8, (n >> 2) & 1, sm.abort_flag(),
+                     status);
+      __syncwarp();
+    }
     tm_fence_after();
   }
   // This warp is past its last load from fill n.
@@ -737,8 +742,7 @@ struct Tm {
             ep += P * kTmRecord;
             if (!more) return;
           }
-          if (!ready) tm_take(sm, u.n, status);
-          tm_fence_after();
+          tm_take(sm, u.n, status, ready);
         }
         load(t + c, b);
       }
