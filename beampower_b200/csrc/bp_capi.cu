@@ -587,10 +587,17 @@ std::vector<Part> parts_of(const bp_table* t, int storage, bool maxred, bool sta
   return parts;
 }
 
+#if BP_DEBUG_CHECKS
+std::atomic<int> g_lose_fill{0};  // LaunchArgs::lose_fill of the next launches
+#endif
+
 // Rows of the max buffer, or the tensor-memory kernel's ring stages.
 void set_fit(bp::LaunchArgs& a, int cfg, int rows) {
   a.red_rows = std::max(1, rows);
   a.n_stage = cfg == kTmemConfig ? rows : 0;
+#if BP_DEBUG_CHECKS
+  a.lose_fill = g_lose_fill.load();
+#endif
 }
 
 // Whether some staged shape serves table `t` with this storage and reduction
@@ -2042,3 +2049,10 @@ int bp_debug_wait_timeout(unsigned long long limit_ns, void* stream, int* status
 }
 
 }  // extern "C"
+
+#if BP_DEBUG_CHECKS
+// Index-checked build only: the tensor-memory kernel's block 0 (of a batch, every
+// block) leaves out a fill, counted from 1 (0: none), so that the waits for it run
+// out.
+extern "C" BP_API void bp_debug_lose_fill(int fill) { g_lose_fill.store(fill); }
+#endif

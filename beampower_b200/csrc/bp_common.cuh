@@ -141,10 +141,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
-// The same for waits that are part of a kernel's rhythm: a tight loop of 4096
+// The same for waits that are part of a kernel's rhythm: a tight loop of kSpin
 // tries between looks at the abort flag and the clock.
 __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity,
                                                volatile int* abort_flag, int* status) {
+  constexpr int kSpin = 64;
   unsigned long long start = 0;
   while (true) {
     uint32_t ok;
@@ -155,13 +156,13 @@ __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity,
         "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
         "@p bra DONE;\n\t"
         "add.u32 n, n, 1;\n\t"
-        "setp.lt.u32 p, n, 4096;\n\t"
+        "setp.lt.u32 p, n, %3;\n\t"
         "@p bra WAIT;\n"
         "DONE:\n\t"
-        "setp.lt.u32 p, n, 4096;\n\t"
+        "setp.lt.u32 p, n, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "n"(kSpin)
         : "memory");
     if (ok) return true;
     if (*abort_flag) return false;
@@ -234,6 +235,19 @@ __device__ __forceinline__ float neg_zero() { return __uint_as_float(gridDim.z <
 
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// The same, and whether any of the threads came with `flag` (one answer for all).
+__device__ __forceinline__ bool named_barrier_or(int id, int nthreads, bool flag) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(id), "r"(nthreads), "r"((uint32_t)flag)
+      : "memory");
+  return any != 0;
 }
 
 __device__ __forceinline__ void red_max_u64(unsigned long long* addr, unsigned long long v) {

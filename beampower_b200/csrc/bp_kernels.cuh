@@ -333,6 +333,9 @@ struct LaunchArgs {
   // rows would not leave room for the table's ring.
   int red_rows;
   int n_stage;  // tensor-memory kernel: ring stages
+#if BP_DEBUG_CHECKS
+  int lose_fill;  // tensor-memory kernel: 1 + a fill that is left out (see Tm::state)
+#endif
   TmLayout tm;  // filled at its launch
   int* status;
 };
