@@ -2007,7 +2007,8 @@ int bp_table_kernel_config(const bp_table* t, int storage, int reduce) {
 int bp_get_kernel_config(int storage, int reduce) {
   if (storage < 0 || storage > 2) return 0;
   const int c = chosen_config(storage, reduce == BP_REDUCE_MAX);
-  return c >= 0 ? c : kTmemConfig;
+  if (c >= 0) return c;
+  return storage == BP_STORAGE_F32 ? -1 : kOrder16[0];
 }
 
 }  // extern "C"

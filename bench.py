@@ -816,7 +816,9 @@ def run_batch(args, local_rank):
         "data": "synthetic",
         "config": {"workload": wl["spec"].name, "windows": len(windows),
                    "storage": args.storage, "graph": True, "persistent_launch": True,
-                   "kernel_config": bp.core.load_library("gpu").bp_get_kernel_config(
+                   # of the table with the widest windows, which decides for the batch
+                   "kernel_config": bp.core.load_library("gpu").bp_table_kernel_config(
+                       max(tables, key=lambda t: t.info["max_spread"]).handle,
                        {"fp32": 0, "bf16": 1, "fp16": 2}[args.storage], 1),
                    "l2": "inputs of every step > L2 (features of 128 windows), no flush"},
         "terms_per_step": terms,

@@ -461,6 +461,9 @@ BP_API int bp_kernel_config_describe(int config, int *sources_per_thread,
 BP_API int bp_kernel_config_shape(int config, int *stations_per_stage,
                                   int *sources_per_block, int *blocks_per_sm);
 BP_API int bp_set_kernel_config(int storage, int reduce, int config);
+/* The chosen config; where none is chosen, the built-in default: config 2 for
+ * 16-bit storage, -1 for FP32, whose default depends on the table (see
+ * bp_table_kernel_config).  Setting the answer again changes nothing. */
 BP_API int bp_get_kernel_config(int storage, int reduce);
 /* The shape a call on this table runs with (storage, reduce): the chosen one
  * when its shared memory and blocks per SM fit the table, else the first
