@@ -876,8 +876,7 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
   cudaStream_t st = as_stream(stream);
   int device = 0;
   BP_CUDA(cudaGetDevice(&device));
-  bp_table* t = new bp_table();
-  std::memset(t, 0, sizeof(*t));
+  bp_table* t = new bp_table();  // scalars and pointers zero
   t->device = device;
   retain_pool(t->device);
   t->stream = st;
