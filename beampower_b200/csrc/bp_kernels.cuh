@@ -318,6 +318,8 @@ struct TmLayout {
 
 struct LaunchArgs {
   TableView tab0;               // plain launch: the table
+  // plain launch: its tile i is the table's tile tile_order[i] (nullptr: i)
+  const int* tile_order;
   RecordView rec0;              // plain launch: the record
   const TableView* tables;      // batch launch: device arrays
   const RecordView* records;
@@ -1155,8 +1157,9 @@ beam_window_kernel(const LaunchArgs a) {
   if (threadIdx.x == 0) St::init_barriers(sm);
   __syncthreads();
   const int n_btiles = a.tab0.n_tiles * St::H;
-  const int btile = blockIdx.x % n_btiles;
+  int btile = blockIdx.x % n_btiles;
   const int chunk = blockIdx.x / n_btiles;
+  if (a.tile_order) btile = a.tile_order[btile / St::H] * St::H + btile % St::H;
   const int tau_first = a.rec0.out0 / St::TT;
   const int tau_end = (a.rec0.out1 + St::TT - 1) / St::TT;
   const int tau0 = tau_first + chunk * a.tiles_per_chunk;

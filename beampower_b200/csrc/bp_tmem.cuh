@@ -975,8 +975,9 @@ beam_tmem_kernel(const __grid_constant__ LaunchArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const typename T::Smem sm{smem, a.tm};
   T::start(sm);
-  const int tile = blockIdx.x % a.tab0.n_tiles;
+  int tile = blockIdx.x % a.tab0.n_tiles;
   const int chunk = blockIdx.x / a.tab0.n_tiles;
+  if (a.tile_order) tile = a.tile_order[tile];
   const int tau_end = (a.rec0.out1 + kTmTile - 1) / kTmTile;
   const int tau0 = a.rec0.out0 / kTmTile + chunk * a.tiles_per_chunk;
   const int tau1 = min(tau0 + a.tiles_per_chunk, tau_end);
@@ -1014,7 +1015,8 @@ __device__ __forceinline__ TmItem tm_item(const LaunchArgs& a, int done) {
   const long long pairs = (long long)a.tab0.n_tiles * n_tau;
   const long long j = pairs * blockIdx.x / gridDim.x + done;
   const long long end = pairs * (blockIdx.x + 1) / gridDim.x;
-  const int tile = (int)(j / n_tau), from = (int)(j - (long long)tile * n_tau);
+  const int i = (int)(j / n_tau), from = (int)(j - (long long)i * n_tau);
+  const int tile = a.tile_order && j < end ? a.tile_order[i] : i;
   return TmItem{tile, first + from, first + from + (int)min(end - j, (long long)(n_tau - from))};
 }
 
