@@ -21,6 +21,7 @@
 #include <utility>
 
 #include <cooperative_groups.h>
+#include <cuda.h>
 
 #include "bp_stats.cuh"
 
@@ -862,6 +863,44 @@ int local_maxima(const float* x, int n, Mask* peaks, Scratch& sc, cudaStream_t s
   return scan_counts(*peaks, st);
 }
 
+// SMs that the blocks of a launch on `st` can have: the device's, or fewer where the
+// stream or the current context has a share of them (a green context).
+int stream_sms(cudaStream_t st, int* sms) {
+  using GetStream = CUresult (*)(CUstream, CUgreenCtx*);
+  using GetGreen = CUresult (*)(CUgreenCtx, CUdevResource*, CUdevResourceType);
+  using GetCtx = CUresult (*)(CUcontext, CUdevResource*, CUdevResourceType);
+  using Current = CUresult (*)(CUcontext*);
+  // the driver's calls by name: the library does not link against it
+  static const auto entry = [](const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion(name, &f, 12040, cudaEnableDefault, &q) != cudaSuccess) {
+      cudaGetLastError();
+      return (void*)nullptr;
+    }
+    return q == cudaDriverEntryPointSuccess ? f : nullptr;
+  };
+  static const auto stream_green = (GetStream)entry("cuStreamGetGreenCtx");
+  static const auto green_share = (GetGreen)entry("cuGreenCtxGetDevResource");
+  static const auto current = (Current)entry("cuCtxGetCurrent");
+  static const auto ctx_share = (GetCtx)entry("cuCtxGetDevResource");
+  int dev = 0;
+  BP_CUDA(cudaGetDevice(&dev));
+  BP_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
+  CUdevResource r{};
+  CUgreenCtx green = nullptr;
+  CUcontext ctx = nullptr;
+  if (stream_green && green_share && stream_green(st, &green) == CUDA_SUCCESS && green) {
+    if (green_share(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+      *sms = std::min(*sms, (int)r.sm.smCount);
+  } else if (current && ctx_share && current(&ctx) == CUDA_SUCCESS && ctx) {
+    if (ctx_share(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+      *sms = std::min(*sms, (int)r.sm.smCount);
+  }
+  *sms = std::max(*sms, 1);
+  return BP_OK;
+}
+
 // The distance rule on the peaks pos[0 .. *d_m - 1] (at most `cap`, on the
 // device): the kept ones as a mask with scanned counts.
 int distance_rule(const float* x, int n, const int* pos, const int* d_m, int cap, double distance,
@@ -879,15 +918,22 @@ int distance_rule(const float* x, int n, const int* pos, const int* d_m, int cap
   BP_TRY(sc.get(&a.kept, cap));
   BP_TRY(sc.get(&a.counters, 6));
   BP_TRY(get_mask(&a.out, n, sc));
-  int dev = 0, sms = 0;
-  BP_CUDA(cudaGetDevice(&dev));
-  BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // one block per SM: they are resident together, and a barrier of few blocks is
-  // the quicker one
-  const unsigned grid = grid_for(cap, kDistThreads, sms);
+  // One block per SM: they are resident together, and a barrier of few blocks is the
+  // quicker one.  Fewer blocks do the same work, so where some limit that was not
+  // asked for (a share of the SMs held another way) refuses them, fewer are tried.
+  int sms = 0;
+  BP_TRY(stream_sms(st, &sms));
+  unsigned grid = grid_for(cap, kDistThreads, sms);
   void* args[] = {&a};
-  BP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(distance_kernel), dim3(grid),
-                                      dim3(kDistThreads), args, 0, st));
+  cudaError_t e = cudaSuccess;
+  while (true) {
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(distance_kernel), dim3(grid),
+                                    dim3(kDistThreads), args, 0, st);
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid == 1) break;
+    cudaGetLastError();
+    grid /= 2;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "launch distance_kernel");
   BP_LAUNCHED("distance_kernel");
   *out = a.out;
   return scan_counts(*out, st);
