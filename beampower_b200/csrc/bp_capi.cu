@@ -385,12 +385,14 @@ size_t planes_bytes(int S, int P, size_t pitch) {
 int fill_planes(int S, int P, int storage, const void* traces, size_t pitch, void* planes,
                 cudaStream_t st) {
   const bool f32 = storage == BP_STORAGE_F32;
-  const long long chunks = bp::tm_plane_rows((long long)pitch) * (f32 ? 4 : 2);
-  const dim3 grid((unsigned)((chunks + 255) / 256), (unsigned)(S * P * (f32 ? 1 : 2)));
+  const dim3 grid((unsigned)bp::tm_planes_blocks((long long)pitch, f32),
+                  (unsigned)(S * P * (f32 ? 1 : 2)));
   const auto* in = static_cast<const uint4*>(traces);
   auto* out = static_cast<uint4*>(planes);
-  if (f32) bp::planes_kernel<true><<<grid, 256, 0, st>>>(in, (long long)pitch, out);
-  else bp::planes_kernel<false><<<grid, 256, 0, st>>>(in, (long long)pitch, out);
+  if (f32)
+    bp::planes_kernel<true><<<grid, bp::kPlanesBlock, 0, st>>>(in, (long long)pitch, out);
+  else
+    bp::planes_kernel<false><<<grid, bp::kPlanesBlock, 0, st>>>(in, (long long)pitch, out);
   BP_LAUNCHED("planes_kernel");
   return BP_OK;
 }
@@ -1585,10 +1587,9 @@ struct bp_batch {
   int red_rows;
   bool checked;
   void* planes;                     // tensor-memory kernel: the records' traces as planes
-  std::vector<size_t> planes_at;    // byte offset of each record's planes
-  std::vector<bp_record> records;   // their traces
-  std::vector<int> record_S;
-  void* mem;                        // device: tables, records, prefix, keys, srcmm, queue, status
+  long long planes_blocks;          // that fill them
+  long long* d_planes_prefix;       // per record
+  void* mem;                        // device: tables, records, prefixes, keys, srcmm, queue, status
   bp::TableView* d_tables;
   bp::RecordView* d_records;
   long long* d_prefix;
@@ -1767,7 +1768,6 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   b->mem = nullptr;
   b->planes = planes;
   planes = nullptr;
-  b->records.assign(records, records + n_records);
   b->stream = st;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -1778,6 +1778,7 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   const size_t o_t = take(n_tables * sizeof(bp::TableView));
   const size_t o_r = take(n_records * sizeof(bp::RecordView));
   const size_t o_p = take((n_records + 1) * sizeof(long long));
+  const size_t o_pp = take((n_records + 1) * sizeof(long long));
   const size_t o_k = take(n_keys * sizeof(unsigned long long));
   const size_t o_m = take(n_srcmm * sizeof(int2));
   const size_t o_q = take(sizeof(unsigned long long));
@@ -1792,6 +1793,7 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   b->d_tables = reinterpret_cast<bp::TableView*>(base + o_t);
   b->d_records = reinterpret_cast<bp::RecordView*>(base + o_r);
   b->d_prefix = reinterpret_cast<long long*>(base + o_p);
+  b->d_planes_prefix = reinterpret_cast<long long*>(base + o_pp);
   b->d_keys = reinterpret_cast<unsigned long long*>(base + o_k);
   b->n_keys = n_keys;
   b->d_queue = reinterpret_cast<unsigned long long*>(base + o_q);
@@ -1802,15 +1804,17 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   };
   // keys and delay ranges inside the allocation
   size_t koff = 0, moff = 0, poff = 0;
+  std::vector<long long> planes_prefix(n_records + 1, 0);
   int2* d_srcmm = reinterpret_cast<int2*>(base + o_m);
   for (int r = 0; r < n_records; ++r) {
     rv[r].keys = b->d_keys + koff;
     if (b->planes) {
       const int S = tables[rv[r].table]->dev.S;
       rv[r].planes = static_cast<const unsigned char*>(b->planes) + poff;
-      b->planes_at.push_back(poff);
-      b->record_S.push_back(S);
       poff += planes_bytes(S, P, records[r].pitch);
+      planes_prefix[r + 1] =
+          planes_prefix[r] + bp::tm_planes_blocks(rv[r].pitch, storage == BP_STORAGE_F32) *
+                                 S * P * (storage == BP_STORAGE_F32 ? 1 : 2);
     }
     koff += (size_t)(rv[r].out1 - rv[r].out0);
     if (records[r].station_mask) {
@@ -1829,9 +1833,13 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->d_prefix, prefix.data(), (n_records + 1) * sizeof(long long),
                         cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(b->d_planes_prefix, planes_prefix.data(),
+                        (n_records + 1) * sizeof(long long), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_status, 0, sizeof(int), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return bail(cuda_fail(e, "batch descriptors"));
+  b->planes_blocks = planes_prefix[n_records];
   *out = b;
   return BP_OK;
 }
@@ -1843,12 +1851,16 @@ int bp_batch_run(bp_batch* b, void* stream) {
   cudaStream_t st = as_stream(stream);
   BP_CUDA(cudaMemsetAsync(b->d_keys, 0, std::max<size_t>(b->n_keys, 1) * 8, st));
   BP_CUDA(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned long long), st));
-  if (b->planes)
-    for (int r = 0; r < b->n_records; ++r)
-      if (int rc = fill_planes(b->record_S[r], b->P, b->storage, b->records[r].traces,
-                               b->records[r].pitch,
-                               static_cast<unsigned char*>(b->planes) + b->planes_at[r], st))
-        return rc;
+  if (b->planes_blocks > 0) {
+    const unsigned grid = (unsigned)b->planes_blocks;
+    if (b->storage == BP_STORAGE_F32)
+      bp::batch_planes_kernel<true>
+          <<<grid, bp::kPlanesBlock, 0, st>>>(b->d_records, b->n_records, b->d_planes_prefix);
+    else
+      bp::batch_planes_kernel<false>
+          <<<grid, bp::kPlanesBlock, 0, st>>>(b->d_records, b->n_records, b->d_planes_prefix);
+    BP_LAUNCHED("batch_planes_kernel");
+  }
   bp::LaunchArgs a{};
   a.tables = b->d_tables;
   a.records = b->d_records;
