@@ -129,6 +129,7 @@ struct bp_table {
   float* weights;    // (N, S), direct kernel only
   int* status;       // kernel status word
   double mean_spread;  // mean span of the used (tile, station, phase) windows
+  double mean_active;  // mean active stations of a tile
   bool real_weights;   // some weight is neither 0 nor 1
   // Tiles in ascending order of their widest window (of tables with windows too
   // wide for the tensor-memory kernel; empty otherwise): its span, and the mean.
@@ -486,26 +487,111 @@ double tmem_limit(const bp_table* t, int storage, bool maxred) {
   if (!maxred) limit -= 30.0;
   return limit;
 }
-bool prefers_tmem(const bp_table* t, int storage, bool maxred) {
-  return t->mean_spread <= tmem_limit(t, storage, maxred);
+// (table tile, time tile) pairs of a launch that is not known yet: many.
+constexpr long long kManyPairs = 1ll << 60;
+
+// Whether the tensor-memory kernel's blocks take equal shares of a launch's pairs
+// (see beam_tmem_share_kernel).  That evens out the last wave and saves the prologue
+// of a block per pair, but a block's share is a run of like tiles, so the tiles have
+// to cost the same: as many active stations in each, two fills in TMEM even of the
+// widest window (`spread`).  The kernel of shares spills with three phases.  Above 32
+// pairs per SM blocks take two pairs and more, and are the better balance as soon as
+// those are some work (active stations x phases x time tiles of a block).
+// Measured as times of the staged kernel over those of blocks | shares (B200; S active
+// stations; us of the staged kernel):
+//   pairs per SM             3            5            12           24           40
+//   S 20, 2 phases   112: 1.18|1.21  187: 1.15|1.26  392: 1.28|1.52  705: 1.20|1.46  1139: 1.39|1.46
+//   S 12, 2 phases    95: 0.94|1.07  128: 1.04|1.25  289: 1.04|1.39  485: 0.93|1.33   765: 1.10|1.30
+//   S 12, 1 phase     70: 0.86|1.03   93: 0.96|1.13  204: 0.95|1.36  327: 0.83|1.23   508: 1.03|1.22
+//   S 40, 1 phase, any weights
+//                    138: 1.14|1.19  237: 1.08|1.26  495: 1.17|1.42  928: 1.10|1.37  1505: 1.25|1.38
+//   S 20, 2 phases, whole response
+//                    104: 1.10|1.13  186: 1.14|1.22  401: 1.22|1.39  716: 1.12|1.31  1149: 1.27|1.29
+//   S 14 of 27, 2 phases
+//                     90: 0.89|0.77  124: 0.92|0.88  275: 0.98|0.93  456: 0.87|0.81   720: 1.01|0.78
+//   S 28 of 37, 2 phases            239: 1.00|0.88  458: 1.08|0.99  833: 1.05|0.97  1391: 1.15|0.95
+//   S 31, 2 phases, windows to 322
+//                    160: 0.89|0.89  236: 0.93|0.86  551: 1.03|0.84  984: 0.98|0.81  1600: 1.07|0.80
+//   S 20, 3 phases   149: 0.98|0.89  256: 1.02|0.89  541: 1.05|0.98  998: 1.01|0.93  1639: 1.10|0.92
+constexpr int kSharePairs = 32;
+bool tmem_two_fills(int spread) { return spread + 16 <= bp::kTmCols / 2; }
+bool equal_tiles(const bp_table* t) {
+  return t->mean_active >= 0.95 * (double)t->info.max_active;
+}
+// Active stations x phases x time tiles of a block, with blocks of a few pairs
+// (choose_tiles_per_chunk).
+double block_work(const bp_table* t, double per_sm) {
+  return std::min(std::max(std::floor(per_sm / 16.0), 1.0), 64.0) * t->mean_active * t->dev.P;
+}
+bool tmem_shares(const bp_table* t, long long pairs, int spread) {
+  const double per_sm = (double)pairs / std::max(1, device_sm_count(t->device));
+  return t->dev.P <= 2 && tmem_two_fills(spread) && equal_tiles(t) &&
+         (per_sm <= kSharePairs || block_work(t, per_sm) < 55.0);
 }
 
-// The caller's choice if it serves this table; else the tensor-memory kernel
-// where it is the faster one; else the first shape of the storage's order
-// that serves the table; config 0 (the smallest) as the last resort.
-// staged_only: non-finite weights under the flexible rule, or no memory for
-// the planes.
-int config_for(const bp_table* t, int storage, bool maxred, bool staged_only = false) {
-  const int c = chosen_config(storage, maxred);
-  if (c >= 0 && !(staged_only && c == kTmemConfig) && config_fits(t, c, storage, maxred))
-    return c;
-  if (!staged_only && prefers_tmem(t, storage, maxred) &&
+// Whether the tensor-memory kernel is the faster one for a launch of `pairs` pairs, of
+// windows that are narrow enough (tmem_limit).  With few pairs its tiles of 64 sources
+// and one block per SM leave SMs idle where the staged shapes have more and smaller
+// blocks: up to 2 pairs per SM it has 0.5 to 1.0 of the staged kernel's speed on every
+// network above (S 60, 1 phase, at 2.7: 1.42 with shares), and with 2 stations 0.88 at 3.
+// Without shares, a block of one pair pays its prologue and the first fills with the
+// stations of one time tile, so it needs some work: more of it where tiles differ, and
+// then the more where the kernel's variant spills (three phases and more) or stores a
+// whole response.  Staged over tensor-memory times on both sides of the lines, by work:
+//   equal tiles
+//   40   work 49 (S 49, 1 phase): 1.13 at 21 pairs per SM; work 43: 1.10 at 5; work 48 (3
+//        phases, any weights): 1.19 at 8; work 60 (3 phases): 1.02, 1.05, 1.01 at 5, 12, 24
+//        work 31 (S 31, 1 phase): 1.05, 1.06, 0.97; work 36 (3 phases): 0.93, 0.91, 0.83
+//   70   (mean span above 100) work 62: 0.93, 1.03, 0.98; at 40 (work 124) 1.07
+//   tiles that differ
+//   55   work 57 (S 28 of 40, 2 phases): 1.04 at 5, 1.09 at 12, 1.03 at 24
+//        work 29 (S 14 of 27, 2 phases): 0.92, 0.98, 0.87; at 40 (work 58) 1.01
+//   80   (whole response) work 57: 0.99, 1.02, 0.96; at 40 (work 114) 1.07; work 58: 0.94
+//   100  (3 phases) work 88: 0.95 at 40
+//   200  (3 phases, whole response) work 88: 0.91 at 40, work 176: 0.96 at 64
+// Whole responses with one fill per TMEM, 2 phases: 0.68 to 0.94 up to 40 pairs per SM.
+bool tmem_pays(const bp_table* t, bool maxred, long long pairs, int spread) {
+  const double sms = std::max(1, device_sm_count(t->device));
+  const double per_sm = (double)pairs / sms;
+  const bool equal = equal_tiles(t);
+  const double work = block_work(t, per_sm);
+  if (tmem_shares(t, pairs, spread))
+    return per_sm >= (work >= 50.0 ? 1.9 : work >= 10.0 ? 2.9 : 5.0);
+  if (!maxred && t->dev.P >= 2 && !tmem_two_fills(spread)) return false;
+  const bool wide = t->mean_spread > 100.0;
+  if (equal) return per_sm >= kSharePairs || (per_sm >= 2.9 && work >= (wide ? 70.0 : 40.0));
+  const double least = t->dev.P > 2 ? (maxred ? 100.0 : 200.0)
+                       : !maxred    ? 80.0
+                       : wide       ? 70.0
+                                    : 55.0;
+  return per_sm >= 5.0 && work >= least;
+}
+bool prefers_tmem(const bp_table* t, int storage, bool maxred, long long pairs) {
+  return t->mean_spread <= tmem_limit(t, storage, maxred) &&
+         tmem_pays(t, maxred, pairs, t->info.max_spread);
+}
+
+// Without a choice of the caller's: the tensor-memory kernel where it is the faster
+// one; else the first shape of the storage's order that serves the table; config 0
+// (the smallest) as the last resort.  staged_only: non-finite weights under the
+// flexible rule, or no memory for the planes.  pairs: (table tile, time tile) pairs of
+// the launch.
+int default_config(const bp_table* t, int storage, bool maxred, bool staged_only,
+                   long long pairs) {
+  if (!staged_only && prefers_tmem(t, storage, maxred, pairs) &&
       config_fits(t, kTmemConfig, storage, maxred))
     return kTmemConfig;
   const int* order = storage == BP_STORAGE_F32 ? kOrderF32 : kOrder16;
   for (int i = 0; i < kStagedConfigs; ++i)
     if (config_fits(t, order[i], storage, maxred)) return order[i];
   return 0;
+}
+
+// The caller's choice if it serves this table, else the default of a long call.
+int config_for(const bp_table* t, int storage, bool maxred) {
+  const int c = chosen_config(storage, maxred);
+  if (c >= 0 && config_fits(t, c, storage, maxred)) return c;
+  return default_config(t, storage, maxred, false, kManyPairs);
 }
 
 // Tiles [tile0, tile0 + n_tiles) of a table, which one launch takes.
@@ -523,15 +609,24 @@ struct Part {
 // pairs (sources x time) per SM, else it goes with the next wider one.
 // (16,000 sources, 60 stations, 60,007 samples, windows of up to 4,300 samples,
 // weights not 0 / 1: 18.5 ms as one launch, 15.8 ms as two.)
-std::vector<Part> parts_of(const bp_table* t, int storage, bool maxred, bool staged_only,
-                           long long n_tt) {
+struct Parts {
+  Part part[3];
+  int n = 0;
+};
+Parts parts_of(const bp_table* t, int storage, bool maxred, bool staged_only, long long n_tt) {
   const int n = t->dev.n_tiles;
-  std::vector<Part> parts;
+  Parts parts;
   const int c = chosen_config(storage, maxred);
-  const bool chosen =
-      c >= 0 && !(staged_only && c == kTmemConfig) && config_fits(t, c, storage, maxred);
   int at = 0;
-  if (!chosen && (int)t->tile_max.size() == n) {
+  auto add = [&](int cfg, int end, int spread) {
+    parts.part[parts.n++] = Part{cfg, at, end - at, spread};
+    at = end;
+  };
+  if (c >= 0 && !(staged_only && c == kTmemConfig) && config_fits(t, c, storage, maxred)) {
+    add(c, n, t->info.max_spread);
+    return parts;
+  }
+  if ((int)t->tile_max.size() == n) {
     const long long least = 32ll * std::max(1, device_sm_count(t->device));
     auto fit = [&](int cfg) {  // tiles that a config serves: a prefix
       int lo = 0, hi = n;
@@ -542,30 +637,25 @@ std::vector<Part> parts_of(const bp_table* t, int storage, bool maxred, bool sta
       }
       return lo;
     };
-    auto add = [&](int cfg, int end) {
-      if ((long long)(end - at) * n_tt < least) return;
-      parts.push_back(Part{cfg, at, end - at, t->tile_max[end - 1]});
-      at = end;
-    };
     if (!staged_only) {
       const double limit = tmem_limit(t, storage, maxred);
       int narrow = 0;
       for (int i = 0; i < n; ++i) narrow += t->tile_mean[i] <= limit;
-      add(kTmemConfig, std::min(narrow, fit(kTmemConfig)));
+      const int end = std::min(narrow, fit(kTmemConfig));
+      if (end * n_tt >= least && tmem_pays(t, maxred, end * n_tt, t->tile_max[end - 1]))
+        add(kTmemConfig, end, t->tile_max[end - 1]);
     }
     const int* order = storage == BP_STORAGE_F32 ? kOrderF32 : kOrder16;
     for (int i = 0; at < n && i < kStagedConfigs; ++i) {
       const int end = fit(order[i]);
       if (end - at < (n - at + 1) / 2) continue;
-      if (end < n) add(order[i], end);
+      if (end < n && (end - at) * n_tt >= least) add(order[i], end, t->tile_max[end - 1]);
       break;
     }
   }
-  if (at < n) {
-    const int cfg = at == 0 ? config_for(t, storage, maxred, staged_only)
-                            : config_for(t, storage, maxred, true);
-    parts.push_back(Part{cfg, at, n - at, t->info.max_spread});
-  }
+  if (at < n)
+    add(default_config(t, storage, maxred, staged_only || at > 0, n * n_tt), n,
+        t->info.max_spread);
   return parts;
 }
 
@@ -626,19 +716,15 @@ bp::TableView table_view(const bp_table* t) {
   return v;
 }
 
-// Up to this many (table tile, time tile) pairs per SM the tensor-memory kernel's
-// blocks take equal shares of them (see beam_tmem_share_kernel).
-constexpr long long kSharePairs = 16;
-
 // The launches of a plain call: a.rec0 is its record (planes not set).
 int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bool checked,
               cudaStream_t st) {
   bp::RecordView& r = a.rec0;
   const int whole = 32 * 16;
   const long long n_tt = (r.out1 + whole - 1) / whole - r.out0 / whole;
-  std::vector<Part> parts = parts_of(t, storage, maxred, checked, n_tt);
+  Parts parts = parts_of(t, storage, maxred, checked, n_tt);
   PlanesScratch planes;
-  if (n_tt > 0 && !parts.empty() && parts[0].cfg == kTmemConfig) {
+  if (n_tt > 0 && parts.n > 0 && parts.part[0].cfg == kTmemConfig) {
     const size_t pitch = (size_t)r.pitch;
     if (planes.get(planes_bytes(t->dev.S, t->dev.P, pitch), st)) {
       if (int rc = fill_planes(t->dev.S, t->dev.P, storage, r.traces, pitch, planes.p, st))
@@ -650,7 +736,8 @@ int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bo
   }
   a.max_active = std::max(1, t->info.max_active);
   a.status = t->status;
-  for (const Part& p : parts) {
+  for (int i = 0; i < parts.n; ++i) {
+    const Part& p = parts.part[i];
     const int tt = cfg_time_tile(p.cfg);
     const int n_tau = (r.out1 + tt - 1) / tt - r.out0 / tt;
     if (n_tau <= 0) return BP_OK;
@@ -663,10 +750,10 @@ int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bo
     set_fit(a, p.cfg, rows_for(t, p.cfg, storage, maxred, p.spread));
     long long blocks =
         (long long)((n_tau + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
-    const int sms = std::max(1, device_sm_count(t->device));
-    if (p.cfg == kTmemConfig && (long long)n_tau * n_btiles <= kSharePairs * sms) {
+    const long long pairs = (long long)n_tau * n_btiles;
+    if (p.cfg == kTmemConfig && tmem_shares(t, pairs, p.spread)) {
       a.tiles_per_chunk = 0;
-      blocks = std::min<long long>((long long)n_tau * n_btiles, sms);
+      blocks = std::min<long long>(pairs, std::max(1, device_sm_count(t->device)));
     }
     const int rc = maxred ? launch_window<true>(p.cfg, t->dev.P, checked, storage, a, false,
                                                 blocks, t->device, st)
@@ -961,6 +1048,7 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
     std::memcpy(&sum, stats + bp::kStatSpreadSum, 8);
     t->real_weights = stats[bp::kStatReal] != 0;
     t->mean_spread = rows ? (double)sum / (double)rows : 0.0;
+    t->mean_active = n_tiles > 0 ? (double)rows / (double)(P * (size_t)n_tiles) : 0.0;
   }
   // The staged kernel serves the table when some shape holds its windows
   // with FP32 storage (the smallest ring).  16-bit storage keeps four copies
@@ -1649,11 +1737,19 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   const int chosen = chosen_config(storage, true);
   if (!checked && P >= 1 && P <= 4 && (chosen < 0 || chosen == kTmemConfig)) {
     bool tmem = true;
+    // the records' (table tile, time tile) pairs; at most kBatchSamplesPerItem samples
+    // of a tile go through a block at a time, so a batch is like a plain launch of
+    // that many pairs
+    long long pairs = 0;
+    for (int r = 0; r < n_records; ++r)
+      if (records[r].table >= 0 && records[r].table < n_tables && tables[records[r].table])
+        pairs += (long long)tables[records[r].table]->dev.n_tiles *
+                 ((long long)(records[r].n_samples + bp::kTmTile - 1) / bp::kTmTile);
     int S = 0, spread = 0, active = 1;
     for (int j = 0; j < n_tables && tmem; ++j) {
       const bp_table* t = tables[j];
       tmem = t && staged_serves(t, storage, true) && t->dev.P == P && t->device == dev &&
-             (chosen == kTmemConfig || prefers_tmem(t, storage, true));
+             (chosen == kTmemConfig || prefers_tmem(t, storage, true, pairs));
       if (!tmem) break;
       S = std::max(S, t->dev.S);
       spread = std::max(spread, t->info.max_spread);

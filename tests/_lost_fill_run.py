@@ -54,7 +54,7 @@ def main():
     # block 0 alone has the first samples
     for storage in ("fp32", "fp16"):
         code = {"fp32": 0, "fp16": 2}[storage]
-        for N, T, fill in ((64, 700, 4), (50, 300 * TILE, fills + 3),
+        for N, T, fill in ((64, 700, 4), (50, 500 * TILE, fills + 3),
                            (64, 4800 * TILE, fills + 1)):
             F, A, D, W = problem(N, T, T)
             table = TravelTimeTable(D, W)
@@ -98,6 +98,7 @@ def main():
             for red in (0, 1):
                 lib.bp_set_kernel_config(code, red, -1)
 
+    lib.bp_set_kernel_config(0, 1, CONFIG)
     # a call that reads the kernel's status says so
     F, A, D, W = problem(64, 700, 1)
     try:
