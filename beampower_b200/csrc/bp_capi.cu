@@ -1709,9 +1709,12 @@ int masked_minmax(const bp::TableView& tv, int P, const uint32_t* mask, int2* ou
 
 extern "C" {
 
-int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record* records,
-                    int n_records, int storage, void* stream, bp_batch** out) {
+// *planes_taken: memory for the records' planes was asked for and given.
+static int batch_create(const bp_table* const* tables, int n_tables, const bp_record* records,
+                        int n_records, int storage, void* stream, bool staged_only,
+                        bool* planes_taken, bp_batch** out) {
   g_last_error.clear();
+  *planes_taken = false;
   if (!out) return fail(BP_ERR_INVALID_ARGUMENT, "out_batch is NULL");
   *out = nullptr;
   if (!tables || n_tables <= 0 || !records || n_records <= 0)
@@ -1735,7 +1738,7 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   int n_stage = 0;
   void* planes = nullptr;
   const int chosen = chosen_config(storage, true);
-  if (!checked && P >= 1 && P <= 4 && (chosen < 0 || chosen == kTmemConfig)) {
+  if (!staged_only && !checked && P >= 1 && P <= 4 && (chosen < 0 || chosen == kTmemConfig)) {
     bool tmem = true;
     // the records' (table tile, time tile) pairs; at most kBatchSamplesPerItem samples
     // of a tile go through a block at a time, so a batch is like a plain launch of
@@ -1766,6 +1769,7 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
         n_stage = 0;
         cudaGetLastError();
       }
+      *planes_taken = planes != nullptr;
     }
   }
   struct PlanesGuard {  // until the batch owns them
@@ -1938,6 +1942,19 @@ int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record
   b->planes_blocks = planes_prefix[n_records];
   *out = b;
   return BP_OK;
+}
+
+int bp_batch_create(const bp_table* const* tables, int n_tables, const bp_record* records,
+                    int n_records, int storage, void* stream, bp_batch** out) {
+  bool planes = false;
+  int rc = batch_create(tables, n_tables, records, n_records, storage, stream, false, &planes,
+                        out);
+  // the planes took what the batch cannot do without: it runs without them
+  if (rc == BP_ERR_OUT_OF_MEMORY && planes) {
+    cudaGetLastError();
+    rc = batch_create(tables, n_tables, records, n_records, storage, stream, true, &planes, out);
+  }
+  return rc;
 }
 
 int bp_batch_run(bp_batch* b, void* stream) {
