@@ -232,6 +232,12 @@ __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b, float neg0) {
 }
 // Grids of these kernels have no z dimension: 1 << 31.
 __device__ __forceinline__ float neg_zero() { return __uint_as_float(gridDim.z << 31); }
+// The same, made anew where it is used: it holds no register elsewhere.
+__device__ __forceinline__ float neg_zero_here() {
+  uint32_t v;
+  asm volatile("{\n\t.reg .u32 z;\n\tmov.u32 z, %%nctaid.z;\n\tshl.b32 %0, z, 31;\n\t}" : "=r"(v));
+  return __uint_as_float(v);
+}
 
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

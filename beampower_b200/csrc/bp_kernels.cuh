@@ -1127,6 +1127,10 @@ struct Staged {
               // stations, 60,007 samples: 16.8 ms scalar, 15.1 ms in pairs with
               // config 8, 19.6 and 18.3 ms with config 1)
               const float2 w2 = make_float2(w, w);
+              // 16 samples per lane and more: a register held for it through the
+              // whole loop spills others, which costs unit weights (config 1 on
+              // wide windows, 6,240 sources, 47 stations: 361 us, 331 so)
+              const float neg0 = MT >= 16 ? neg_zero_here() : neg_zero();
 #pragma unroll
               for (int p = 0; p < P; ++p)
 #pragma unroll
@@ -1134,7 +1138,7 @@ struct Staged {
                   const int q = g0 / 2 + qq;
                   acc[k][q] = add2_rn(
                       acc[k][q],
-                      mul2_rn(w2, make_float2(u[p][2 * qq], u[p][2 * qq + 1]), neg_zero()));
+                      mul2_rn(w2, make_float2(u[p][2 * qq], u[p][2 * qq + 1]), neg0));
                 }
             }
           }
