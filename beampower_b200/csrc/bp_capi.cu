@@ -1074,6 +1074,8 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(t->weights, d_weights, N * S * sizeof(float), cudaMemcpyDeviceToDevice,
                           st);
+    // done before the table is used, on whatever stream
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return bail(cuda_fail(e, "copy table arrays"));
   }
   *out = t;

@@ -62,3 +62,31 @@ def test_used_at_once_on_another_stream(cuda, bplib, oracle_lib, widths):
         assert np.array_equal(am.cpu().numpy(), want[1])
         table.close()
     probe.close()
+
+
+def test_direct_table_used_at_once_on_another_stream(cuda, bplib, oracle_lib):
+    """Five phases: the direct kernel, over the table's copies of the delays."""
+    import torch
+    from beampower_b200.tables import TravelTimeTable
+    S, P, N, T = 20, 5, 40_000, 600
+    rng = np.random.default_rng(7)
+    D = rng.integers(0, 200, size=(N, S, P)).astype(np.int32)
+    W = np.ones((N, S), np.float32)
+    F = rng.standard_normal((S, 1, T)).astype(np.float32)
+    A = rng.uniform(0.2, 1.2, size=(S, 1, P)).astype(np.float32)
+    want = oracle_lib.beamform_max(oracle_lib.prestack(F, A), D, W, 1)
+    d, w = torch.from_numpy(D).cuda(), torch.from_numpy(W).cuda()
+    probe = TravelTimeTable(d, w)
+    assert probe.info["uses_window_kernel"] == 0
+    traces = probe.traces_from_features(F, A)
+    made, used = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        table = TravelTimeTable(d, w, stream=made)
+        with torch.cuda.stream(used):
+            bm, am = table.beamform_max(traces, 1, stream=used)
+        used.synchronize()
+        assert np.array_equal(_bits(bm.cpu().numpy()), _bits(want[0]))
+        assert np.array_equal(am.cpu().numpy(), want[1])
+        table.close()
+    probe.close()
