@@ -571,6 +571,17 @@ bool prefers_tmem(const bp_table* t, int storage, bool maxred, long long pairs) 
          tmem_pays(t, maxred, pairs, t->info.max_spread);
 }
 
+// The same for the table of a batch, whose kernel takes items from a queue and spills
+// more.  Times of the batch on staged shape 8 over the tensor-memory kernel's (10 windows
+// of 6,000 samples; by stations, mean span; 50,000 sources and less):
+//   2 phases, weights 0 / 1: S 40, 71: 1.67, S 60, 102: 1.25, S 30, 109: 0.98, S 100, 112:
+//   1.08, S 88, 125: 0.78, S 94, 137: 0.54; any weights: S 40, 89: 1.21
+//   1 phase: S 40, 59: 1.71, any weights 1.26;  3 phases: S 60, 34: 0.95, S 40, 79: 0.86;
+//   4 phases: S 40, 39: 1.65
+bool batch_prefers_tmem(const bp_table* t, int storage, long long pairs) {
+  return t->dev.P != 3 && t->mean_spread <= 105.0 && prefers_tmem(t, storage, true, pairs);
+}
+
 // Without a choice of the caller's: the tensor-memory kernel where it is the faster
 // one; else the first shape of the storage's order that serves the table; config 0
 // (the smallest) as the last resort.  staged_only: non-finite weights under the
@@ -1754,7 +1765,7 @@ static int batch_create(const bp_table* const* tables, int n_tables, const bp_re
     for (int j = 0; j < n_tables && tmem; ++j) {
       const bp_table* t = tables[j];
       tmem = t && staged_serves(t, storage, true) && t->dev.P == P && t->device == dev &&
-             (chosen == kTmemConfig || prefers_tmem(t, storage, true, pairs));
+             (chosen == kTmemConfig || batch_prefers_tmem(t, storage, pairs));
       if (!tmem) break;
       S = std::max(S, t->dev.S);
       spread = std::max(spread, t->info.max_spread);

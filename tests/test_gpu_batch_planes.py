@@ -64,3 +64,32 @@ def test_records_of_unlike_lengths(cuda, bplib, oracle_lib, forced, storage):
     assert counts == [one + (one - 3) * (len(LENGTHS) - 1)] * 2
     few.close()
     table.close()
+
+
+@pytest.mark.parametrize("P,width,tmem", [(2, 30, True), (2, 139, False), (3, 30, False)])
+def test_choice(cuda, bplib, oracle_lib, P, width, tmem):
+    """Tables of narrow and of wide mean windows, and of three phases."""
+    import torch
+    from beampower_b200.batch import Window, WindowBatch
+    from beampower_b200.core import launch_count
+    from beampower_b200.tables import TravelTimeTable
+    rng = np.random.default_rng(P + width)
+    S, T = 20, 512 * 20
+    D = rng.integers(0, width, size=(64 * 40, S, P)).astype(np.int32)
+    W = np.ones(D.shape[:2], np.float32)
+    A = rng.uniform(0.2, 1.2, size=(S, 1, P)).astype(np.float32)
+    F = rng.standard_normal((S, 1, T)).astype(np.float32)
+    table = TravelTimeTable(D, W)
+    batch = WindowBatch([table], [Window(0, T)], A, storage="fp32")
+    batch.set_features(0, F)
+    before = launch_count()
+    (bm, am), = batch.run()
+    assert launch_count() - before == (4 if tmem else 3)  # prestack, planes, beams, decode
+    torch.cuda.synchronize()
+    n = 600
+    want = oracle_lib.beamform_max(oracle_lib.prestack(
+        np.ascontiguousarray(F[:, :, :n + width]), A), D, W, 0)
+    assert np.array_equal(bm[:n].cpu().numpy().view(np.uint32), want[0][:n].view(np.uint32))
+    assert np.array_equal(am[:n].cpu().numpy(), want[1][:n])
+    batch.close()
+    table.close()
