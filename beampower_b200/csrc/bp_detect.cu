@@ -88,6 +88,37 @@ __device__ __forceinline__ void pw_up(float& v, bool h, unsigned lanes, int o) {
   if (has) v = __fadd_rn(v, r);
 }
 
+// A leaf's sum by eight lanes (`lane` of them, `group` their mask), one of its eight
+// strided partial sums each; adding the partial sums by exchange is NumPy's order,
+// since a rounded addition commutes.  get(i): value i.  All lanes of the group call it.
+template <class Get>
+__device__ __forceinline__ float pw_leaf(const PwNode& nd, int lane, unsigned group,
+                                         const Get& get) {
+  float r = 0.0f;
+  if (nd.len >= 8) {
+    // the lane's values and the leaf's tail, loaded before they are added
+    const int rows = nd.len / 8, tail = nd.len % 8, lim = nd.begin + nd.len - tail;
+    float v[kPwLeaf / 8], t[7];
+#pragma unroll
+    for (int i = 0; i < kPwLeaf / 8; ++i) v[i] = i < rows ? get(nd.begin + 8 * i + lane) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) t[i] = i < tail ? get(lim + i) : 0.0f;
+    r = v[0];
+#pragma unroll
+    for (int i = 1; i < kPwLeaf / 8; ++i)
+      if (i < rows) r = __fadd_rn(r, v[i]);
+    r = __fadd_rn(r, __shfl_xor_sync(group, r, 1));
+    r = __fadd_rn(r, __shfl_xor_sync(group, r, 2));
+    r = __fadd_rn(r, __shfl_xor_sync(group, r, 4));
+#pragma unroll
+    for (int i = 0; i < 7; ++i)
+      if (i < tail) r = __fadd_rn(r, t[i]);
+  } else {
+    for (int i = 0; i < nd.len; ++i) r = __fadd_rn(r, get(nd.begin + i));
+  }
+  return r;
+}
+
 // The sum of `count` (a power of two) paths' nodes at their common root: a warp
 // for 32 of them at a time, in shared memory.
 __device__ float pw_join(float* val, unsigned char* has, int count) {
@@ -115,9 +146,7 @@ __device__ float pw_join(float* val, unsigned char* has, int count) {
 // `root`) of segments of `len` values that start every seg_stride values, as
 // NumPy's mean / var store them.  Block (b, w) sums the 1 << lower paths below
 // path b of the upper `upper` turns of segment w's tree, and the last of a
-// segment's blocks joins their sums.  Eight lanes take a leaf, one of its eight
-// strided partial sums each; adding the partial sums by exchange is NumPy's
-// order, since a rounded addition commutes.
+// segment's blocks joins their sums.
 // What bounds it is latency: on 2.16 million samples a launch takes 13 us where
 // a thread per leaf and a second launch for the inner nodes, level by level from
 // tables in global memory, took 46.
@@ -152,29 +181,7 @@ pw_kernel(const float* __restrict__ x, long long seg_stride, int len, int n_seg,
                          : PwNode{0, 0};
       __syncthreads();
       const PwNode nd = nodes[tid / 8];
-      float r = 0.0f;
-      if (nd.len >= 8) {
-        // the lane's values and the leaf's tail, loaded before they are added
-        const int rows = nd.len / 8, tail = nd.len % 8, lim = nd.begin + nd.len - tail;
-        float v[kPwLeaf / 8], t[7];
-#pragma unroll
-        for (int i = 0; i < kPwLeaf / 8; ++i)
-          v[i] = i < rows ? get(nd.begin + 8 * i + lane) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 7; ++i) t[i] = i < tail ? get(lim + i) : 0.0f;
-        r = v[0];
-#pragma unroll
-        for (int i = 1; i < kPwLeaf / 8; ++i)
-          if (i < rows) r = __fadd_rn(r, v[i]);
-        r = __fadd_rn(r, __shfl_xor_sync(group, r, 1));
-        r = __fadd_rn(r, __shfl_xor_sync(group, r, 2));
-        r = __fadd_rn(r, __shfl_xor_sync(group, r, 4));
-#pragma unroll
-        for (int i = 0; i < 7; ++i)
-          if (i < tail) r = __fadd_rn(r, t[i]);
-      } else {
-        for (int i = 0; i < nd.len; ++i) r = __fadd_rn(r, get(nd.begin + i));
-      }
+      float r = pw_leaf(nd, lane, group, get);
       __syncwarp();
       const bool h = nd.len > 0;
       pw_up(r, h, kFull, 8);  // the warp's four leaves
@@ -214,10 +221,68 @@ pw_kernel(const float* __restrict__ x, long long seg_stride, int len, int n_seg,
   }
 }
 
+// The same for segments of at most 1 << kPwShort leaves: a block takes as many of them
+// as its 64 groups of eight lanes have leaves for.  (With a block of pw_kernel for each,
+// the threshold of 2.16 million samples over windows of 500 took 564 us and over windows
+// of 7 took 22.4 ms; now 142 and 230, and 256 and 1,232 with a thread per leaf.)
+constexpr int kPwShort = 6, kPwShortThreads = 8 << kPwShort;
+__global__ void __launch_bounds__(kPwShortThreads)
+pw_short_kernel(const float* __restrict__ x, long long seg_stride, int len, int n_seg, int mode,
+                const float* __restrict__ centre, int depth, bool root,
+                float* __restrict__ out) {
+  __shared__ float val[kPwShortThreads / 32];
+  __shared__ unsigned char has[kPwShortThreads / 32];
+  const int tid = threadIdx.x, slot = tid / 8;
+  const int each = 1 << (kPwShort - depth);  // segments of a block
+  const int w = blockIdx.x * each + (slot >> depth);
+  const bool live = w < n_seg;
+  const float* base = x + (size_t)(live ? w : 0) * seg_stride;
+  const float c = mode && live ? centre[w] : 0.0f;
+  PwNode nd{0, live ? len : 0};
+  if (live) nd = nd.down(slot & ((1 << depth) - 1), depth);
+  float r = pw_leaf(nd, tid & 7, 0xFFu << (tid & 24), [&](int i) {
+    const float v = base[i];
+    if (!mode) return v;
+    const float d = __fsub_rn(v, c);
+    return __fmul_rn(d, d);
+  });
+  __syncwarp();
+  const bool h = nd.len > 0;
+  if (depth >= 1) pw_up(r, h, kFull, 8);  // the warp's four leaves
+  if (depth >= 2) pw_up(r, h, kFull, 16);
+  const int lane = tid & 31;
+  bool write = (lane & ((8 << min(depth, 2)) - 1)) == 0;
+  int mine = w;
+  if (depth > 2) {  // then the warps
+    if (lane == 0) {
+      val[tid / 32] = r;
+      has[tid / 32] = h;
+    }
+    __syncthreads();
+    if (tid >= 32) return;
+    const bool g = lane < kPwShortThreads / 32 && has[lane];
+    r = g ? val[lane] : 0.0f;
+    for (int o = 1; o < 1 << (depth - 2); o *= 2) pw_up(r, g, kFull, o);
+    write = lane < kPwShortThreads / 32 && (lane & ((1 << (depth - 2)) - 1)) == 0;
+    mine = blockIdx.x * each + (lane >> (depth - 2));
+  }
+  if (write && mine < n_seg) {
+    const float v = np_divide_count(__fadd_rn(0.0f, r), len);
+    out[mine] = root ? __fsqrt_rn(v) : v;
+  }
+}
+
 // tickets: n_seg zeros, for this call alone.
 int pw_mean(const float* x, long long seg_stride, int len, int n_seg, int mode,
             const float* centre, bool root, float* out, Scratch& sc, cudaStream_t st) {
   const int depth = pw_depth(len);
+  if (depth <= kPwShort && n_seg > 1) {
+    const int each = 1 << (kPwShort - depth);
+    pw_short_kernel<<<(unsigned)(((long long)n_seg + each - 1) / each), kPwShortThreads, 0, st>>>(
+        x, seg_stride, len, n_seg, mode, centre, depth, root, out);
+    BP_LAUNCHED("pw_short_kernel");
+    return BP_OK;
+  }
   // 128 leaves per block, at most 256 blocks per segment, at most 4,096 leaves
   // per block: 2.16 million samples have 32,768
   const int lower = std::min(std::max(std::min(depth, 7), depth - 8), 12), upper = depth - lower;
