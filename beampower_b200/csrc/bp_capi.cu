@@ -1037,6 +1037,24 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
     rc = build_tiles(d_delays, d_weights, t->dev, st);
     if (rc) return bail(rc);
   }
+  // The direct kernel reads the raw arrays: it gets private copies, which are done
+  // before the table is used, on whatever stream.
+  auto copy_arrays = [&]() -> int {
+    cudaError_t c = cudaMallocAsync(
+        &t->direct_mem, N * S * P * sizeof(int32_t) + N * S * sizeof(float) + 256, st);
+    if (c != cudaSuccess) return cuda_fail(c, "cudaMallocAsync(table copies)");
+    t->delays = reinterpret_cast<int32_t*>(t->direct_mem);
+    t->weights = reinterpret_cast<float*>(
+        reinterpret_cast<char*>(t->direct_mem) + pad256(N * S * P * sizeof(int32_t)));
+    c = cudaMemcpyAsync(t->delays, d_delays, N * S * P * sizeof(int32_t),
+                        cudaMemcpyDeviceToDevice, st);
+    if (c == cudaSuccess)
+      c = cudaMemcpyAsync(t->weights, d_weights, N * S * sizeof(float), cudaMemcpyDeviceToDevice,
+                          st);
+    return c == cudaSuccess ? BP_OK : cuda_fail(c, "copy table arrays");
+  };
+  if (!window && N > 0)  // waited for with the statistics
+    if (int rc2 = copy_arrays()) return bail(rc2);
   int stats[bp::kStatCount];
   e = cudaMemcpyAsync(stats, t->dev.stats, sizeof(stats), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1072,22 +1090,10 @@ static int table_create_based(const int32_t* d_delays, const float* d_weights, s
   // parts_of
   if (use_window && n_tiles > 1 && !config_fits(t, kTmemConfig, BP_STORAGE_F32, true))
     if (int rc2 = order_tiles(t, st)) return bail(rc2);
-  if (!use_window && N > 0) {
-    // The direct kernel reads the raw arrays: keep private copies.
-    e = cudaMallocAsync(&t->direct_mem, N * S * P * sizeof(int32_t) + N * S * sizeof(float) + 256,
-                        st);
-    if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMallocAsync(table copies)"));
-    t->delays = reinterpret_cast<int32_t*>(t->direct_mem);
-    t->weights = reinterpret_cast<float*>(
-        reinterpret_cast<char*>(t->direct_mem) + pad256(N * S * P * sizeof(int32_t)));
-    e = cudaMemcpyAsync(t->delays, d_delays, N * S * P * sizeof(int32_t),
-                        cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(t->weights, d_weights, N * S * sizeof(float), cudaMemcpyDeviceToDevice,
-                          st);
-    // done before the table is used, on whatever stream
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return bail(cuda_fail(e, "copy table arrays"));
+  if (window && !use_window && N > 0) {
+    if (int rc2 = copy_arrays()) return bail(rc2);
+    if (cudaError_t c = cudaStreamSynchronize(st); c != cudaSuccess)
+      return bail(cuda_fail(c, "copy table arrays"));
   }
   *out = t;
   return BP_OK;
