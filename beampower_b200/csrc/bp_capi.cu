@@ -549,7 +549,10 @@ bool tmem_shares(const bp_table* t, long long pairs, int spread) {
 //   80   (whole response) work 57: 0.99, 1.02, 0.96; at 40 (work 114) 1.07; work 58: 0.94
 //   100  (3 phases) work 88: 0.95 at 40
 //   200  (3 phases, whole response) work 88: 0.91 at 40, work 176: 0.96 at 64
-// Whole responses with one fill per TMEM, 2 phases: 0.68 to 0.94 up to 40 pairs per SM.
+// Whole responses of 2 phases with windows that leave TMEM one fill (some tiles do):
+//   equal tiles, S 40, mean span 65: 1.06 at 12, 1.20 at 41, 1.21 at 99 pairs per SM; 78:
+//   1.01, 1.11, 1.12; 90: 0.95, 1.03, 1.04; 103: 0.93, 1.01, 1.03; 115: 0.83, 0.91, 0.92
+//   tiles that differ, S 28 of 40, 59: 0.85, 0.95, 0.96; S 28 of 37, 96: 0.81, 0.94, 0.87
 bool tmem_pays(const bp_table* t, bool maxred, long long pairs, int spread) {
   const double sms = std::max(1, device_sm_count(t->device));
   const double per_sm = (double)pairs / sms;
@@ -557,7 +560,9 @@ bool tmem_pays(const bp_table* t, bool maxred, long long pairs, int spread) {
   const double work = block_work(t, per_sm);
   if (tmem_shares(t, pairs, spread))
     return per_sm >= (work >= 50.0 ? 1.9 : work >= 10.0 ? 2.9 : 5.0);
-  if (!maxred && t->dev.P >= 2 && !tmem_two_fills(spread)) return false;
+  if (!maxred && t->dev.P >= 2 && !tmem_two_fills(spread) &&
+      (!equal || t->mean_spread > (per_sm >= kSharePairs ? 105.0 : 80.0)))
+    return false;
   const bool wide = t->mean_spread > 100.0;
   if (equal) return per_sm >= kSharePairs || (per_sm >= 2.9 && work >= (wide ? 70.0 : 40.0));
   const double least = t->dev.P > 2 ? (maxred ? 100.0 : 200.0)
