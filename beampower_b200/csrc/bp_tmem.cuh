@@ -890,8 +890,9 @@ struct Tm {
     const int src0 = warp * KS;
     const int4* my_src = sm.srci() + src0;
     const int own = 16 * lane;
+    int past = 0;  // moves the loop beyond its end
 #pragma unroll 1
-    for (int tau = tau0; tau < tau1; ++tau) {
+    for (int tau = tau0; tau + past < tau1; ++tau) {
       const int t0 = tau * kTmTile;
       float2 acc[KS][8];  // pair x: samples own + 2x, + 1
 #pragma unroll
@@ -953,9 +954,10 @@ struct Tm {
         }
         // A warp whose wait ran out (which raised the abort flag) has summed what
         // was not there: none of them writes, and all of them end with this tile.
-        // (Leaving the loop from here instead spills 39 registers of its body.)
+        // (Leaving the loop from here spills 39 registers of its body, and setting
+        // its end costs the form with shares and one phase 12%.)
         const bool lost = named_barrier_or(1, kTmCompute * 32, *sm.abort_flag() != 0);
-        if (lost) tau1 = tau;
+        if (lost) past = 1 << 30;
         {
           const unsigned long long* r0 = reinterpret_cast<const unsigned long long*>(sm.red()) +
                                          (tid & 15) * 33 + (tid >> 4);
@@ -969,13 +971,18 @@ struct Tm {
         named_barrier_sync(1, kTmCompute * 32);
       } else {
         // (a wait of this warp that ran out raised the abort flag)
-        if (__any_sync(0xFFFFFFFFu, *sm.abort_flag() != 0)) break;
+        // (the two ways out: with one phase setting `past` costs the form with shares
+        // 13%, with two and three the other one 10 to 40%)
+        if (__any_sync(0xFFFFFFFFu, *sm.abort_flag() != 0)) {
+          if constexpr (P == 1) break;
+          past = 1 << 30;
+        }
         // through this warp's buffer, so that the stores are coalesced
         float* buf = reinterpret_cast<float*>(sm.red()) + warp * (16 * 34);
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
           const int4 si = my_src[k];
-          if (si.x < 0) continue;  // warp-uniform
+          if (si.x < 0 || past) continue;  // warp-uniform
           float* out = rc.beam + (size_t)si.x * rc.ldb - rc.out0;
 #pragma unroll
           for (int x = 0; x < 16; ++x)
