@@ -494,9 +494,10 @@ constexpr long long kManyPairs = 1ll << 60;
 // (see beam_tmem_share_kernel).  That evens out the last wave and saves the prologue
 // of a block per pair, but a block's share is a run of like tiles, so the tiles have
 // to cost the same: as many active stations in each, two fills in TMEM even of the
-// widest window (`spread`).  The kernel of shares spills with three phases.  Above 32
-// pairs per SM blocks take two pairs and more, and are the better balance as soon as
-// those are some work (active stations x phases x time tiles of a block).
+// widest window (`spread`).  Whole responses of three phases and more have no gain (0.9
+// of the blocks' speed).  Above 32 pairs per SM blocks take two pairs and more, and are
+// the better balance as soon as those are some work (active stations x phases x time
+// tiles of a block).
 // Measured as times of the staged kernel over those of blocks | shares (B200; S active
 // stations; us of the staged kernel):
 //   pairs per SM             3            5            12           24           40
@@ -512,28 +513,40 @@ constexpr long long kManyPairs = 1ll << 60;
 //   S 28 of 37, 2 phases            239: 1.00|0.88  458: 1.08|0.99  833: 1.05|0.97  1391: 1.15|0.95
 //   S 31, 2 phases, windows to 322
 //                    160: 0.89|0.89  236: 0.93|0.86  551: 1.03|0.84  984: 0.98|0.81  1600: 1.07|0.80
-//   S 20, 3 phases   149: 0.98|0.89  256: 1.02|0.89  541: 1.05|0.98  998: 1.01|0.93  1639: 1.10|0.92
+//   S 20, 3 phases   147: 0.99|1.02  256: 1.02|1.04  544: 1.05|1.15  844: 1.00|1.10
+//   S 20, 4 phases   221: 1.10|1.23  392: 1.10|1.24  843: 1.16|1.38  1337: 1.12|1.34
+//   (the last column of these two at 20)
+// With tiles that differ a little (mean over most active stations 0.84 to 0.95; same
+// order, shares only): 1 phase 0.97 at 3, 1.09 at 5, 1.33 at 12, 1.24 at 30; 2 phases 1.05,
+// 1.13, 1.34; 3 phases 0.85, 0.88, 0.97, 0.93.  With 0.65 to 0.84 and 1 phase 0.94 at 5, 1.04
+// to 1.11 at 8 and 12, 0.98 at 20.
 constexpr int kSharePairs = 32;
 bool tmem_two_fills(int spread) { return spread + 16 <= bp::kTmCols / 2; }
-bool equal_tiles(const bp_table* t) {
-  return t->mean_active >= 0.95 * (double)t->info.max_active;
+// How alike the tiles' numbers of active stations are: 1 when they are equal.
+double evenness(const bp_table* t) {
+  return t->info.max_active > 0 ? t->mean_active / (double)t->info.max_active : 1.0;
 }
 // Active stations x phases x time tiles of a block, with blocks of a few pairs
 // (choose_tiles_per_chunk).
 double block_work(const bp_table* t, double per_sm) {
   return std::min(std::max(std::floor(per_sm / 16.0), 1.0), 64.0) * t->mean_active * t->dev.P;
 }
-bool tmem_shares(const bp_table* t, long long pairs, int spread) {
+bool tmem_shares(const bp_table* t, bool maxred, long long pairs, int spread) {
+  const int P = t->dev.P;
   const double per_sm = (double)pairs / std::max(1, device_sm_count(t->device));
-  return t->dev.P <= 2 && tmem_two_fills(spread) && equal_tiles(t) &&
-         (per_sm <= kSharePairs || block_work(t, per_sm) < 55.0);
+  const double even = evenness(t);
+  if (!tmem_two_fills(spread) || (!maxred && P > 2)) return false;
+  if (even >= 0.95) return per_sm <= kSharePairs || block_work(t, per_sm) < 55.0;
+  if (even >= 0.84) return P <= 2 && per_sm <= kSharePairs;
+  return even >= 0.65 && P == 1 && per_sm >= 8.0 && per_sm <= 16.0;
 }
 
 // Whether the tensor-memory kernel is the faster one for a launch of `pairs` pairs, of
 // windows that are narrow enough (tmem_limit).  With few pairs its tiles of 64 sources
 // and one block per SM leave SMs idle where the staged shapes have more and smaller
 // blocks: up to 2 pairs per SM it has 0.5 to 1.0 of the staged kernel's speed on every
-// network above (S 60, 1 phase, at 2.7: 1.42 with shares), and with 2 stations 0.88 at 3.
+// network above (S 60, 1 phase, at 2.7: 1.42 with shares), and with little work in a pair
+// (active stations x phases) at 3 too: work 2 0.88, 4 0.93, 8 1.08 at 3.8, 16 1.12 at 2.9.
 // Without shares, a block of one pair pays its prologue and the first fills with the
 // stations of one time tile, so it needs some work: more of it where tiles differ, and
 // then the more where the kernel's variant spills (three phases and more) or stores a
@@ -543,32 +556,46 @@ bool tmem_shares(const bp_table* t, long long pairs, int spread) {
 //        phases, any weights): 1.19 at 8; work 60 (3 phases): 1.02, 1.05, 1.01 at 5, 12, 24
 //        work 31 (S 31, 1 phase): 1.05, 1.06, 0.97; work 36 (3 phases): 0.93, 0.91, 0.83
 //   70   (mean span above 100) work 62: 0.93, 1.03, 0.98; at 40 (work 124) 1.07
-//   tiles that differ
-//   55   work 57 (S 28 of 40, 2 phases): 1.04 at 5, 1.09 at 12, 1.03 at 24
-//        work 29 (S 14 of 27, 2 phases): 0.92, 0.98, 0.87; at 40 (work 58) 1.01
-//   80   (whole response) work 57: 0.99, 1.02, 0.96; at 40 (work 114) 1.07; work 58: 0.94
+//   150  (4 phases, whose staged shapes spill most) work 160: 1.35 at 0.7, 1.11 at 1.5
+//   tiles that differ (evenness 0.65 and more, less)
+//   42   work 45 (S 22 of 30, 1 phase): 1.10 at 34; work 51 (S 26 of 30, 2 phases): 1.10 at
+//        5, 1.19 at 12, 1.14 at 30; work 57 (S 28 of 40, 2 phases): 1.04, 1.09, 1.03
+//        work 30 (S 30 of 40, 1 phase): 0.97, 1.01, 0.93
+//   55   work 29 (S 14 of 27, 2 phases): 0.92, 0.98, 0.87; at 40 (work 58) 1.01
+//   55, 80  (whole response) work 57: 1.04 at 5, 1.07 at 12, 1.00 at 20; work 56 (S 28 of 37,
+//        1 phase): 1.08 at 33; work 58 (S 14 of 27): 0.97 at 33, 1.04 at 64 (work 116)
+//   70   (3 phases, evenness 0.84 and more) work 76: 1.05 at 5, 1.09 at 12, 1.05 at 30
 //   100  (3 phases) work 88: 0.95 at 40
 //   200  (3 phases, whole response) work 88: 0.91 at 40, work 176: 0.96 at 64
 // Whole responses of 2 phases with windows that leave TMEM one fill (some tiles do):
 //   equal tiles, S 40, mean span 65: 1.06 at 12, 1.20 at 41, 1.21 at 99 pairs per SM; 78:
 //   1.01, 1.11, 1.12; 90: 0.95, 1.03, 1.04; 103: 0.93, 1.01, 1.03; 115: 0.83, 0.91, 0.92
-//   tiles that differ, S 28 of 40, 59: 0.85, 0.95, 0.96; S 28 of 37, 96: 0.81, 0.94, 0.87
+//   tiles that differ, S 28 of 37, 96: 1.07 at 11, 1.01 at 22, 1.10 at 33, 1.14 at 66
 bool tmem_pays(const bp_table* t, bool maxred, long long pairs, int spread) {
   const double sms = std::max(1, device_sm_count(t->device));
   const double per_sm = (double)pairs / sms;
-  const bool equal = equal_tiles(t);
+  const int P = t->dev.P;
+  const double even = evenness(t);
   const double work = block_work(t, per_sm);
-  if (tmem_shares(t, pairs, spread))
-    return per_sm >= (work >= 50.0 ? 1.9 : work >= 10.0 ? 2.9 : 5.0);
-  if (!maxred && t->dev.P >= 2 && !tmem_two_fills(spread) &&
-      (!equal || t->mean_spread > (per_sm >= kSharePairs ? 105.0 : 80.0)))
+  if (tmem_shares(t, maxred, pairs, spread)) {
+    const double from = even < 0.95                          ? (P == 1 ? 4.0 : 3.0)
+                        : P > 3 && work >= 150.0             ? 0.5
+                        : P > 3 || (P < 3 && work >= 50.0) ? 1.9
+                        : work >= 10.0                       ? 2.8
+                        : work >= 4.0                        ? 3.5
+                                                             : 5.0;
+    return per_sm >= from;
+  }
+  if (!maxred && P >= 2 && !tmem_two_fills(spread) &&
+      (even < 0.65 || t->mean_spread > (per_sm >= kSharePairs ? 105.0 : 80.0)))
     return false;
   const bool wide = t->mean_spread > 100.0;
-  if (equal) return per_sm >= kSharePairs || (per_sm >= 2.9 && work >= (wide ? 70.0 : 40.0));
-  const double least = t->dev.P > 2 ? (maxred ? 100.0 : 200.0)
-                       : !maxred    ? 80.0
-                       : wide       ? 70.0
-                                    : 55.0;
+  if (even >= 0.95)
+    return per_sm >= kSharePairs || (P > 3 && work >= 150.0 && per_sm >= 0.5) ||
+           (per_sm >= 2.9 && work >= (wide ? 70.0 : 40.0));
+  double least = wide ? 70.0 : even >= 0.65 ? 42.0 : 55.0;
+  if (!maxred) least = even >= 0.65 ? 55.0 : 80.0;
+  if (P > 2) least = !maxred ? 200.0 : even >= 0.84 ? 70.0 : 100.0;
   return per_sm >= 5.0 && work >= least;
 }
 bool prefers_tmem(const bp_table* t, int storage, bool maxred, long long pairs) {
@@ -767,7 +794,7 @@ int run_parts(const bp_table* t, bp::LaunchArgs& a, int storage, bool maxred, bo
     long long blocks =
         (long long)((n_tau + a.tiles_per_chunk - 1) / a.tiles_per_chunk) * n_btiles;
     const long long pairs = (long long)n_tau * n_btiles;
-    if (p.cfg == kTmemConfig && tmem_shares(t, pairs, p.spread)) {
+    if (p.cfg == kTmemConfig && tmem_shares(t, maxred, pairs, p.spread)) {
       a.tiles_per_chunk = 0;
       blocks = std::min<long long>(pairs, std::max(1, device_sm_count(t->device)));
     }
