@@ -79,6 +79,26 @@ def parse():
     return ap.parse_args()
 
 
+TMEM_CONFIG = 9
+TMEM_WORDS = 136  # 4-byte words per clock and SM that loads alone read from tensor memory
+
+
+def operand_roofline(config, achieved_gbs, smem_gbs, clocks, sms=148):
+    """The roof of the memory that a beam kernel's operands come from: tensor
+    memory for config 9, shared memory (peak measured live) for the staged shapes."""
+    if config != TMEM_CONFIG:
+        peak, bound = smem_gbs, "smem"
+        note = "shared-memory operand roof, peak measured live by bp_measure_peaks"
+    else:
+        mhz = (clocks or {}).get("sm_mhz") or 1965.0
+        peak, bound = TMEM_WORDS * 4 * sms * mhz * 1e6 / 1e9, "tmem"
+        note = ("tensor-memory operand roof: 136 words per clock and SM, measured with loads "
+                "alone (78 with the adds and fills beside them), at the run's clock; of the "
+                "shared-memory roof of the staged shapes: %.2f" % (achieved_gbs / smem_gbs))
+    return {"bound": bound, "achieved": achieved_gbs, "peak": peak, "unit": "GB/s",
+            "frac": achieved_gbs / peak, "note": note}
+
+
 def large_config(N, S, P, T, out_of_bounds, storage):
     """The `config` of the large workload, the same in both arms."""
     return {"workload": LARGE.name, "n_sources": N, "n_stations": S, "n_phases": P,
@@ -507,6 +527,8 @@ def run_ours(args, rank, world, local_rank):
     prestack_ms = statistics.mean(r[1].elapsed_time(r[2]) for r in recs)
     kernel_ms = statistics.mean(r[2].elapsed_time(r[3]) for r in recs)
     info = recs[0][4].info
+    kernel_config = lib.bp_table_kernel_config(
+        recs[0][4].handle, {"fp32": 0, "bf16": 1, "fp16": 2}[args.storage], 1)
     # the other trace storage types on the same resident table (kernel only)
     variants = {}
     run_variants = {}
@@ -605,9 +627,11 @@ def run_ours(args, rank, world, local_rank):
 
     line = None
     if rank == 0:
-        # roofline of the dominant kernel: shared-memory operand delivery,
-        # 4 B of trace per effective term
-        smem_achieved = eff * 4 / (kernel_ms * 1e-3) / 1e9
+        # roofline of the dominant kernel: delivery of its operands, 4 B of
+        # trace per effective term (2 B of 16-bit storage)
+        word = 4 if args.storage == "fp32" else 2
+        roofline = operand_roofline(kernel_config, eff * word / (kernel_ms * 1e-3) / 1e9,
+                                    smem_gbs.value, clocks)
         traffic = None
         if os.path.exists(PROFILE_TRAFFIC):
             with open(PROFILE_TRAFFIC) as fh:
@@ -637,16 +661,9 @@ def run_ours(args, rank, world, local_rank):
             "breakdown_ms": {"table_build": table_ms, "prestack": prestack_ms,
                              "beam_kernel_and_decode": kernel_ms},
             "roofline": {
-                "bound": "smem",
-                "achieved": smem_achieved,
-                "peak": smem_gbs.value,
-                "unit": "GB/s",
-                "frac": smem_achieved / smem_gbs.value,
+                **roofline,
                 "traffic": traffic,
-                "note": "shared-memory operand roof (4 B of trace per effective term), peak "
-                        "measured live by bp_measure_peaks; above 1 where the operands "
-                        "come from tensor memory (kernel config 9), whose own roof is 136 "
-                        "words per clock and SM; FP32 and HBM views below",
+                "kernel_config": kernel_config,
                 "fp32_view": {"achieved_tflops": eff * 2 / (kernel_ms * 1e-3) / 1e12,
                               "peak_tflops": fp32_tf.value},
                 "hbm_view": {"achieved_gbs": hbm_bytes / (ms_per_step * 1e-3) / 1e9,

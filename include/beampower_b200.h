@@ -215,12 +215,13 @@ typedef struct bp_record {
 
 typedef struct bp_batch bp_batch;
 
-/* One record alone (no batch): the plain staged launch over the record's
- * output range, global time origin included; this is what a streamed chunk
- * with its carried samples uses.  d_keys: (out1 - out0) uint64 scratch,
- * cleared here.  station_mask must be NULL.  Stream-ordered; the traces are
- * rearranged into stream-ordered scratch (cudaMallocAsync) where the table
- * runs the tensor-memory kernel; no synchronisation. */
+/* One record alone (no batch): the plain launch over the record's output
+ * range, global time origin included; this is what a streamed chunk with its
+ * carried samples uses.  d_keys: (out1 - out0) uint64 scratch, cleared here.
+ * station_mask must be NULL.  Stream-ordered, no synchronisation; scratch
+ * from cudaMallocAsync where 16-bit traces are expanded and where the
+ * tensor-memory kernel runs (it rearranges the traces), which in a captured
+ * graph becomes allocation nodes. */
 BP_API int bp_record_beamform_max_dev(const bp_table *table, const bp_record *record,
                                       int storage, unsigned long long *d_keys,
                                       void *stream);
@@ -302,9 +303,7 @@ BP_API int bp_beamform_differential_dev(const float *d_traces, size_t n_samples,
  * results (float32 arithmetic in NumPy's own order, SciPy's peak rules).
  * Each allocates its scratch with cudaMallocAsync on `stream` and
  * synchronises `stream` (it reads counts back), so none of them can be
- * captured in a CUDA graph.  bp_threshold_dev keeps the pairwise-sum split
- * tree of each length it has seen on the device (cudaMalloc, up to 64 lengths
- * per process, freed at exit). */
+ * captured in a CUDA graph. */
 
 #define BP_THRESHOLD_RMS 0 /* window mean + num_dev * standard deviation */
 #define BP_THRESHOLD_MAD 1 /* window median + num_dev * median |x - median| */
@@ -441,14 +440,15 @@ BP_API int bp_keys_from_shared_dev(const unsigned long long *d_keys, size_t n_sa
  * lane, consumer warps, ring stages, stations per ring stage, sources per
  * block, blocks per SM), all over the same 64-source tables.  The last config
  * is the tensor-memory kernel, the built-in default of FP32 storage where a
- * table's delay windows are narrow (bp_table_kernel_config tells); it takes
- * stream-ordered scratch of about the traces' size (batches: for their
- * lifetime), and the staged kernel runs where there is no memory for it.
+ * table's delay windows are narrow (bp_table_kernel_config tells) and a call
+ * has enough sources and samples to fill the GPU; it takes stream-ordered
+ * scratch of about the traces' size (batches: for their lifetime), and the
+ * staged kernel runs where there is no memory for it.
  * bp_set_kernel_config chooses one per (storage, reduce) for every later
  * launch in the process (-1: built-in default); the environment variable
  * BEAMPOWER_B200_KERNEL_CONFIG overrides it.  beampower_b200/autotune.py
- * times the shapes on a workload and stores its choices.  A shape whose
- * shared memory does not fit a table falls back to config 0 for that table.
+ * times the shapes on a workload and stores its choices.  A table that the
+ * chosen shape does not fit runs with its built-in default.
  * No reference counterpart (the reference has one launch shape,
  * beamform.cu:10). */
 BP_API int bp_kernel_config_count(void);
@@ -465,10 +465,12 @@ BP_API int bp_set_kernel_config(int storage, int reduce, int config);
  * 16-bit storage, -1 for FP32, whose default depends on the table (see
  * bp_table_kernel_config).  Setting the answer again changes nothing. */
 BP_API int bp_get_kernel_config(int storage, int reduce);
-/* The shape a call on this table runs with (storage, reduce): the chosen one
- * when its shared memory and blocks per SM fit the table, else the first
- * that fits in a fixed, measured order (of a table whose tiles run as several
- * launches, without a chosen shape: the widest tiles'); -1 when no shape holds the table's
+/* The shape a long call on this table runs with (storage, reduce): the chosen
+ * one when its shared memory and blocks per SM fit the table, else the
+ * tensor-memory kernel where it is the faster one (calls of few sources and
+ * samples take a staged shape instead), else the first that fits in a fixed,
+ * measured order (of a table whose tiles run as several launches, without a
+ * chosen shape: the widest tiles'); -1 when no shape holds the table's
  * windows in this storage (16-bit calls then expand their traces to FP32 and
  * run the FP32 shape, with the direct kernel's values, when that fits; else,
  * and for tables with uses_window_kernel == 0, the direct kernel runs); a
